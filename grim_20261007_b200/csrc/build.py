@@ -16,7 +16,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 SOURCES = ['grimgpu.cu']
-HEADERS = ['common.cuh', 'hankel.cuh', 'fill2d.cuh', 'linalg.cuh', 'lu.cuh', 'tc_gemm.cuh', 'ozaki.cuh', 'dmma.cuh',
+HEADERS = ['common.cuh', 'hankel.cuh', 'hankel64.cuh', 'fill2d.cuh', 'linalg.cuh', 'lu.cuh', 'tc_gemm.cuh', 'ozaki.cuh', 'dmma.cuh',
            'grouped.cuh', 'farblock.cuh', 'galerkin.cuh', 'pivot.cuh', 'condest.cuh', 'bor.cuh', 'noalloc.cu',
            'tslu.cuh', 'gepp_loop.cuh', 'modecond.cuh']
 OUT = os.path.join(PKG, 'libgrimgpu.so')

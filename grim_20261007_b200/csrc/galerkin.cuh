@@ -41,6 +41,7 @@
 
 #include "common.cuh"
 #include "hankel.cuh"
+#include "hankel64.cuh"
 
 #define GAL_FAR_RATIO 3.0
 #define GAL_EPS 1e-12
@@ -53,10 +54,11 @@
 #define GAL_SUB_KL 2.0
 #define GAL_TILE 32
 #define GAL_FAR_THREADS 256
+#define GAL_FAR_LANES 8
+#define GAL_FAR_SUMS 26
+#define GAL_FAR_SMEM ((size_t)GAL_FAR_SUMS * GAL_FAR_THREADS * sizeof(double))
 #define GAL_NEAR_WARPS 4
 #define GAL_LOAD_ORDER 8
-#define GAL_X_ASYM 25.0
-#define GAL_ASYM64_TERMS 16
 
 #define GAL_ROUTE_SELF 0
 #define GAL_ROUTE_TOUCH 1
@@ -68,11 +70,6 @@
 struct GalElem {
     double ax, ay, bx, by, nx, ny, len, pad;
 };
-
-// Hankel asymptotic coefficients a_k(0), a_k(1), k < GAL_ASYM64_TERMS (DLMF 10.17.1),
-// uploaded with the other tables.
-__constant__ double c_gal_a0[GAL_ASYM64_TERMS];
-__constant__ double c_gal_a1[GAL_ASYM64_TERMS];
 
 __device__ __forceinline__ GalElem gal_load(const double *elem, int e) {
     const double2 *p = (const double2 *)(elem + 8 * (size_t)e);
@@ -239,67 +236,15 @@ __global__ void k_gal_near_list(int ne, const double *__restrict__ elem, const i
     }
 }
 
-// ------------------------------------------------------------------ Hankel functions
-// (j/4) H0^(2)(x) and (j/4) k H1^(2)(x) for real x > 0.
-//   x >= GAL_X_ASYM: H_nu^(2)(x) = sqrt(2/(pi x)) (P_nu - j Q_nu) e^{-j(x - nu pi/2 - pi/4)},
-//   P_nu = sum_m (-1)^m a_2m(nu) x^-2m, Q_nu = sum_m (-1)^m a_2m+1(nu) x^-2m-1 (DLMF 10.17.3),
-//   16 terms: the first omitted term is below 3e-16 of the sum at x = 25;
-//   below: CUDA's double-precision j0, y0, j1, y1.
-// Asymptotic branch with the first TERMS coefficients (TERMS even).
-template <int TERMS>
-__device__ __forceinline__ void gal_hankel_asym(double x, double k, double2 &g, double2 &hk) {
-    const double inv = 1.0 / x;
-    const double inv2 = inv * inv;
-    // Horner in inv2 from the highest even / odd coefficient down
-    double p0 = 0.0, q0 = 0.0, p1 = 0.0, q1 = 0.0;
-#pragma unroll
-    for (int m = TERMS / 2 - 1; m >= 0; --m) {
-        const double sg = (m & 1) ? -1.0 : 1.0;
-        p0 = fma(p0, inv2, sg * c_gal_a0[2 * m]);
-        q0 = fma(q0, inv2, sg * c_gal_a0[2 * m + 1]);
-        p1 = fma(p1, inv2, sg * c_gal_a1[2 * m]);
-        q1 = fma(q1, inv2, sg * c_gal_a1[2 * m + 1]);
-    }
-    q0 *= inv;
-    q1 *= inv;
-    double sx, cx;
-    sincos(x, &sx, &cx);
-    // C = sqrt(2/(pi x)) e^{-j(x - pi/4)}, e^{-j(x - pi/4)} = ((c + s) - j (s - c)) / sqrt(2)
-    const double amp = sqrt(inv * (1.0 / GRIM_PI));  // sqrt(2/(pi x)) / sqrt(2)
-    const double cr = amp * (cx + sx), ci = -amp * (sx - cx);
-    // g = (1/4)(Q0 + j P0) C ; hk = -(k/4)(P1 - j Q1) C
-    g = make_double2(0.25 * (q0 * cr - p0 * ci), 0.25 * (q0 * ci + p0 * cr));
-    const double kq = -0.25 * k;
-    hk = make_double2(kq * (p1 * cr + q1 * ci), kq * (p1 * ci - q1 * cr));
-}
-
-// G and its normal-derivative factor at x = k r.  Above GAL_X_ASYM the DLMF 10.17 expansion,
-// with as many terms as the argument needs for double precision (measured against SciPy's
-// Hankel functions, worst of orders 0 and 1: 16 terms 2.8e-15 at x = 25; 12 terms 3e-15 at
-// x = 35; 8 terms 8.5e-15 at x = 80, where the phase rounding already dominates); below it
-// CUDA's j0 / y0 / j1 / y1.
-__device__ __forceinline__ void gal_hankel(double x, double k, double2 &g, double2 &hk) {
-    if (x >= 80.0) {
-        gal_hankel_asym<8>(x, k, g, hk);
-    } else if (x >= 35.0) {
-        gal_hankel_asym<12>(x, k, g, hk);
-    } else if (x >= GAL_X_ASYM) {
-        gal_hankel_asym<GAL_ASYM64_TERMS>(x, k, g, hk);
-    } else {
-        const double j0v = j0(x), y0v = y0(x), j1v = j1(x), y1v = y1(x);
-        // (j/4)(J0 - j Y0) = (Y0 + j J0)/4 ; (j/4) k (J1 - j Y1) = (k/4)(Y1 + j J1)
-        g = make_double2(0.25 * y0v, 0.25 * j0v);
-        hk = make_double2(0.25 * k * y1v, 0.25 * k * j1v);
-    }
-}
-
-// Near-pair kernel values: r floored at GAL_EPS and k r at 1e-12 (the reference's floors).
+// Near-pair kernel values (j/4) H0^(2)(k r) and (j/4) k H1^(2)(k r): r floored at GAL_EPS and
+// k r at 1e-12 (the reference's floors).
 __device__ __forceinline__ void gal_hankel_near(double r, double k, double2 &g, double2 &hk) {
     double x = k * fmax(r, GAL_EPS);
     if (fabs(x) <= 1e-12) x = 1e-12;
-    const double j0v = j0(x), y0v = y0(x), j1v = j1(x), y1v = y1(x);
-    g = make_double2(0.25 * y0v, 0.25 * j0v);
-    hk = make_double2(0.25 * k * y1v, 0.25 * k * j1v);
+    hankel_pair(x * x, g, hk);
+    const double sc = k * x;
+    hk.x *= sc;
+    hk.y *= sc;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -841,35 +786,13 @@ __device__ __forceinline__ int gal_far_order(double kl_max, double ratio_min, in
 
 #define GAL_MAX_Q 16
 
-// Far pairs of one 32 x 32 tile of the upper tile triangle (rows ti <= cols tj); pairs
-// e < f only on diagonal tiles.  One set of Hankel evaluations per pair gives both
-// orientations: E[e][f] and E[f][e].  min_order: the floor on the tile order (the TE rows'
-// W rule: 8, or 16 outside its calibration; 0 for TM).
-// Two CTAs per SM (at most 128 registers a thread): 16 warps hide the FP64 latency of the
-// Hankel evaluations better than 8 (the accumulators of the pair spill a few words).
-template <int POL, typename C>
-__global__ void __launch_bounds__(GAL_FAR_THREADS, 2)
-k_gal_far(int ne, const double *__restrict__ elem, const int2 *__restrict__ nodes, double k, int min_order,
-          C *__restrict__ E) {
-    const int ti = blockIdx.y, tj = blockIdx.x;
-    if (ti > tj) return;
-    __shared__ GalElem so[GAL_TILE], ss[GAL_TILE];
-    __shared__ int2 sno[GAL_TILE], sns[GAL_TILE];
+// Gauss order of one 32 x 32 tile from its worst far pair, the same in every thread; 0 when
+// the tile has no far pair.
+__device__ __forceinline__ int gal_tile_order(int ne, int e0, int f0, const GalElem *so, const GalElem *ss,
+                                              const int2 *sno, const int2 *sns, double k, int min_order) {
     __shared__ double red_r[GAL_FAR_THREADS / 32], red_l[GAL_FAR_THREADS / 32];
-    __shared__ double qt[GAL_MAX_Q], qw[GAL_MAX_Q];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int e0 = ti * GAL_TILE, f0 = tj * GAL_TILE;
-    if (tid < GAL_TILE) {
-        const int e = min(e0 + tid, ne - 1), f = min(f0 + tid, ne - 1);
-        so[tid] = gal_load(elem, e);
-        ss[tid] = gal_load(elem, f);
-        sno[tid] = nodes[e];
-        sns[tid] = nodes[f];
-    }
-    __syncthreads();
-    // tile order from its worst far pair
     double rmin = INFINITY, lmax = 0.0;
-    for (int p = tid; p < GAL_TILE * GAL_TILE; p += GAL_FAR_THREADS) {
+    for (int p = threadIdx.x; p < GAL_TILE * GAL_TILE; p += GAL_FAR_THREADS) {
         const int le = p & (GAL_TILE - 1), lf = p >> 5;
         const int e = e0 + le, f = f0 + lf;
         if (e < ne && f < ne) {
@@ -882,77 +805,175 @@ k_gal_far(int ne, const double *__restrict__ elem, const int2 *__restrict__ node
         rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
         lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
     }
-    if (lane == 0) {
-        red_r[warp] = rmin;
-        red_l[warp] = lmax;
+    if ((threadIdx.x & 31) == 0) {
+        red_r[threadIdx.x >> 5] = rmin;
+        red_l[threadIdx.x >> 5] = lmax;
     }
     __syncthreads();
-    if (tid == 0) {
-        double r = INFINITY, l = 0.0;
-        for (int w = 0; w < GAL_FAR_THREADS / 32; ++w) {
-            r = fmin(r, red_r[w]);
-            l = fmax(l, red_l[w]);
+#pragma unroll
+    for (int w = 0; w < GAL_FAR_THREADS / 32; ++w) {
+        rmin = fmin(rmin, red_r[w]);
+        lmax = fmax(lmax, red_l[w]);
+    }
+    if (!(rmin < INFINITY)) return 0;
+    return min(GAL_MAX_Q, max(min_order, gal_far_order(fabs(k) * lmax, rmin, 8)));
+}
+
+// Far pairs of the 32 x 32 tiles of the upper tile triangle (rows ti <= cols tj; pairs e < f
+// only on diagonal tiles), gridDim.z CTAs per tile.  One set of Hankel evaluations per pair
+// gives both orientations: E[e][f] and E[f][e].  min_order: the floor on the tile order (the
+// TE rows' W rule: 8, or 16 outside its calibration; 0 for TM).
+//
+// Bound by the FP64 pipe: about 85 FP64 operations a point.  r . n_s does not depend on the
+// point of the (straight) source element and r . n_o not on the observation point, so the
+// normal-derivative kernels of both orientations come from the moments of H1/x against
+// {phi_0^2, phi_0 phi_1, phi_1^2} on either side (phi_a times the linear function with end
+// values d_0, d_1 is d_0 phi_a phi_0 + d_1 phi_a phi_1): six sums a point instead of eight
+// products and eight sums, and no cancellation (every weight is positive).
+// The running sums wait in shared memory, so that 128 registers hold two interleaved points
+// (each coefficient load serves both).  N = 2048, TE (8 x 8 points): 1.37 ms at 59 % of the
+// FP64 pipe, against 2.50 ms with four library Bessel calls a point.
+// LANES threads share a pair, taking every LANES-th observation point each: 8 where one
+// thread per pair would leave the chip idle (N = 333: 0.10 ms, 0.80 ms with one), else 1.
+template <int POL, typename C, int LANES>
+__global__ void __launch_bounds__(GAL_FAR_THREADS, 2)
+k_gal_far(int ne, const double *__restrict__ elem, const int2 *__restrict__ nodes, double k, int min_order,
+          C *__restrict__ E) {
+    const int ti = blockIdx.y, tj = blockIdx.x;
+    if (ti > tj) return;
+    __shared__ GalElem so[GAL_TILE], ss[GAL_TILE];
+    __shared__ int2 sno[GAL_TILE], sns[GAL_TILE];
+    extern __shared__ double gal_far_acc[];  // [GAL_FAR_SUMS][GAL_FAR_THREADS]
+    __shared__ double2 qtab[GAL_MAX_Q + 1][3];  // (t, w phi_0), (w phi_1, w phi_0^2), (w phi_0 phi_1, w phi_1^2)
+    const int tid = threadIdx.x;
+    const int e0 = ti * GAL_TILE, f0 = tj * GAL_TILE;
+    if (tid < GAL_TILE) {
+        const int e = min(e0 + tid, ne - 1), f = min(f0 + tid, ne - 1);
+        so[tid] = gal_load(elem, e);
+        ss[tid] = gal_load(elem, f);
+        sno[tid] = nodes[e];
+        sns[tid] = nodes[f];
+    }
+    __syncthreads();
+    const int q = gal_tile_order(ne, e0, f0, so, ss, sno, sns, k, min_order);
+    if (q == 0) return;  // no far pair in this tile
+    if (tid < q) {
+        double t, w;
+        gal_gauss(q, tid, t, w);
+        const double w1 = w * t, w0 = w - w1, w01 = w1 * (1.0 - t);
+        qtab[tid][0] = make_double2(t, w0);
+        qtab[tid][1] = make_double2(w1, w0 * (1.0 - t));
+        qtab[tid][2] = make_double2(w01, w1 * t);
+        if (tid == q - 1) {  // points are taken in twos: a weightless last one for odd orders
+            qtab[q][0] = make_double2(t, 0.0);
+            qtab[q][1] = qtab[q][2] = make_double2(0.0, 0.0);
         }
-        red_r[0] = r;
-        red_l[0] = l;
     }
-    __syncthreads();
-    if (!(red_r[0] < INFINITY)) return;  // no far pair in this tile
-    const int q = min(GAL_MAX_Q, max(min_order, gal_far_order(fabs(k) * red_l[0], red_r[0], 8)));
-    if (tid < q) gal_gauss(q, tid, qt[tid], qw[tid]);
     __syncthreads();
     const double gi = -1.0 / k;  // gamma = 1/(j k) = -j/k
-    for (int p = tid; p < GAL_TILE * GAL_TILE; p += GAL_FAR_THREADS) {
+    const int sub = tid % LANES;
+    for (int p = (blockIdx.z * GAL_FAR_THREADS + tid) / LANES; p < GAL_TILE * GAL_TILE;
+         p += gridDim.z * (GAL_FAR_THREADS / LANES)) {
         const int le = p & (GAL_TILE - 1), lf = p >> 5;
         const int e = e0 + le, f = f0 + lf;
         if (e >= ne || f >= ne) continue;
         if (ti == tj && e >= f) continue;
-        const GalElem o = so[le], s = ss[lf];
+        const GalElem &o = so[le], &s = ss[lf];
         if (!gal_is_far(o, s, sno[le], sns[lf], e, f)) continue;
-        double S[8], A[8], B[8];  // S; sum h (r.n_s)/r ; sum h (r.n_o)/r  (entries a*2+b, re/im)
+        // running sums in shared memory (one column per thread), so that the registers hold two
+        // points' evaluations at once: 0..7 g against (phi_a, phi_b), 8..25 H1/x against the
+        // quadratics (i, j), re and im
+        double *acc = gal_far_acc + tid;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) S[i] = A[i] = B[i] = 0.0;
-        const double odx = o.bx - o.ax, ody = o.by - o.ay, sdx = s.bx - s.ax, sdy = s.by - s.ay;
-        for (int ip = 0; ip < q; ++ip) {
-            const double tp = qt[ip];
-            const double xpx = o.ax + tp * odx, xpy = o.ay + tp * ody;
-            double rs0x = 0, rs0y = 0, rs1x = 0, rs1y = 0, ra0x = 0, ra0y = 0, ra1x = 0, ra1y = 0;
-            double rb0x = 0, rb0y = 0, rb1x = 0, rb1y = 0;
-            for (int iq = 0; iq < q; ++iq) {
-                const double tq = qt[iq], wq = qw[iq];
-                const double rx = xpx - (s.ax + tq * sdx), ry = xpy - (s.ay + tq * sdy);
-                const double r2 = rx * rx + ry * ry;
-                const double ir = rsqrt(r2);
-                const double r = r2 * ir;
-                double2 g, hk;
-                gal_hankel(k * r, k, g, hk);
-                const double pa = (rx * s.nx + ry * s.ny) * ir, pb = (rx * o.nx + ry * o.ny) * ir;
-                const double w1 = wq * tq, w0 = wq - w1;
-                rs0x = fma(w0, g.x, rs0x); rs0y = fma(w0, g.y, rs0y);
-                rs1x = fma(w1, g.x, rs1x); rs1y = fma(w1, g.y, rs1y);
-                const double hax = hk.x * pa, hay = hk.y * pa, hbx = hk.x * pb, hby = hk.y * pb;
-                ra0x = fma(w0, hax, ra0x); ra0y = fma(w0, hay, ra0y);
-                ra1x = fma(w1, hax, ra1x); ra1y = fma(w1, hay, ra1y);
-                rb0x = fma(w0, hbx, rb0x); rb0y = fma(w0, hby, rb0y);
-                rb1x = fma(w1, hbx, rb1x); rb1y = fma(w1, hby, rb1y);
+        for (int i = 0; i < GAL_FAR_SUMS; ++i) acc[i * GAL_FAR_THREADS] = 0.0;
+        // distances in units of 1/k, from the elements' start points
+        const double bx = k * (o.ax - s.ax), by = k * (o.ay - s.ay);
+        const double odx = k * (o.bx - o.ax), ody = k * (o.by - o.ay);
+        const double sdx = -k * (s.bx - s.ax), sdy = -k * (s.by - s.ay);
+        for (int ip = sub; ip < q; ip += LANES) {
+            const double xpx = fma(qtab[ip][0].x, odx, bx), xpy = fma(qtab[ip][0].x, ody, by);
+            double in[10];  // g against phi_0, phi_1; H1/x against the three quadratics
+#pragma unroll
+            for (int i = 0; i < 10; ++i) in[i] = 0.0;
+#pragma unroll 1
+            for (int iq = 0; iq < q; iq += 2) {
+                double u[2];
+                double2 g[2], h[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const double t = qtab[iq + c][0].x, rx = fma(t, sdx, xpx), ry = fma(t, sdy, xpy);
+                    u[c] = fma(rx, rx, ry * ry);
+                }
+                hankel_pair2(u, g, h);
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const double w0 = qtab[iq + c][0].y;
+                    const double2 s1 = qtab[iq + c][1], s2 = qtab[iq + c][2];
+                    in[0] = fma(w0, g[c].x, in[0]); in[1] = fma(w0, g[c].y, in[1]);
+                    in[2] = fma(s1.x, g[c].x, in[2]); in[3] = fma(s1.x, g[c].y, in[3]);
+                    in[4] = fma(s1.y, h[c].x, in[4]); in[5] = fma(s1.y, h[c].y, in[5]);
+                    in[6] = fma(s2.x, h[c].x, in[6]); in[7] = fma(s2.x, h[c].y, in[7]);
+                    in[8] = fma(s2.y, h[c].x, in[8]); in[9] = fma(s2.y, h[c].y, in[9]);
+                }
             }
-            const double wp = qw[ip];
-            const double v1 = wp * tp, v0 = wp - v1;
-            S[0] = fma(v0, rs0x, S[0]); S[1] = fma(v0, rs0y, S[1]); S[2] = fma(v0, rs1x, S[2]); S[3] = fma(v0, rs1y, S[3]);
-            S[4] = fma(v1, rs0x, S[4]); S[5] = fma(v1, rs0y, S[5]); S[6] = fma(v1, rs1x, S[6]); S[7] = fma(v1, rs1y, S[7]);
-            A[0] = fma(v0, ra0x, A[0]); A[1] = fma(v0, ra0y, A[1]); A[2] = fma(v0, ra1x, A[2]); A[3] = fma(v0, ra1y, A[3]);
-            A[4] = fma(v1, ra0x, A[4]); A[5] = fma(v1, ra0y, A[5]); A[6] = fma(v1, ra1x, A[6]); A[7] = fma(v1, ra1y, A[7]);
-            B[0] = fma(v0, rb0x, B[0]); B[1] = fma(v0, rb0y, B[1]); B[2] = fma(v0, rb1x, B[2]); B[3] = fma(v0, rb1y, B[3]);
-            B[4] = fma(v1, rb0x, B[4]); B[5] = fma(v1, rb0y, B[5]); B[6] = fma(v1, rb1x, B[6]); B[7] = fma(v1, rb1y, B[7]);
-        }
-        const double sc = o.len * s.len;
-        double2 Sb[4], Ab[4], Bb[4];
+            const double2 p0 = qtab[ip][0], p1 = qtab[ip][1], p2 = qtab[ip][2];
+            const double pl[2] = {p0.y, p1.x}, pw[3] = {p1.y, p2.x, p2.y};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            Sb[i] = make_double2(sc * S[2 * i], sc * S[2 * i + 1]);
-            Ab[i] = make_double2(sc * A[2 * i], sc * A[2 * i + 1]);
-            Bb[i] = make_double2(sc * B[2 * i], sc * B[2 * i + 1]);
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    double &v = acc[(4 * a + i) * GAL_FAR_THREADS];
+                    v = fma(pl[a], in[i], v);
+                }
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                    double &v = acc[(8 + 6 * a + i) * GAL_FAR_THREADS];
+                    v = fma(pw[a], in[4 + i], v);
+                }
         }
+        double S[8], R[18];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) S[i] = acc[i * GAL_FAR_THREADS];
+#pragma unroll
+        for (int i = 0; i < 18; ++i) R[i] = acc[(8 + i) * GAL_FAR_THREADS];
+        if (LANES > 1) {
+            const unsigned group = ((1u << LANES) - 1u) << ((tid & 31) & ~(LANES - 1));
+#pragma unroll
+            for (int off = LANES / 2; off > 0; off >>= 1) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) S[i] += __shfl_xor_sync(group, S[i], off);
+#pragma unroll
+                for (int i = 0; i < 18; ++i) R[i] += __shfl_xor_sync(group, R[i], off);
+            }
+            if (sub != 0) continue;
+        }
+        const double sc = o.len * s.len, k2 = k * k * sc;
+        // r . n_s at the observation element's ends, r . n_o at the source element's (times k^2 L_o L_s)
+        const double da0 = k2 * ((o.ax - s.ax) * s.nx + (o.ay - s.ay) * s.ny);
+        const double da1 = k2 * ((o.bx - s.ax) * s.nx + (o.by - s.ay) * s.ny);
+        const double db0 = k2 * ((o.ax - s.ax) * o.nx + (o.ay - s.ay) * o.ny);
+        const double db1 = k2 * ((o.ax - s.bx) * o.nx + (o.ay - s.by) * o.ny);
+        double2 Sb[4], Ab[4], Bb[4];  // S ; sum h (r.n_s)/r ; sum h (r.n_o)/r  (entries a*2+b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int i = 2 * a + b;
+                Sb[i] = make_double2(sc * S[2 * i], sc * S[2 * i + 1]);
+                double v[2], w[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    // phi_a phi_m on the observation side, phi_b = phi_b phi_0 + phi_b phi_1 on the other
+                    v[c] = da0 * (R[6 * a + 2 * b + c] + R[6 * a + 2 * b + 2 + c]) +
+                           da1 * (R[6 * a + 6 + 2 * b + c] + R[6 * a + 6 + 2 * b + 2 + c]);
+                    w[c] = db0 * (R[6 * a + 2 * b + c] + R[6 * a + 6 + 2 * b + c]) +
+                           db1 * (R[6 * a + 2 * b + 2 + c] + R[6 * a + 6 + 2 * b + 2 + c]);
+                }
+                Ab[i] = make_double2(v[0], v[1]);
+                Bb[i] = make_double2(w[0], w[1]);
+            }
         double2 ef[4], fe[4];  // E[e][f][a][b] ; E[f][e][b][a] stored at index a*2+b
         if (POL == GRIM_POL_TM) {
             // E_ef = S + gamma D_ef, D_ef = A ; E_fe[b][a] = S[a][b] + gamma D_fe[b][a], D_fe[b][a] = -B[a][b]

@@ -104,15 +104,9 @@ static int upload_tables(int device) {
     }
     GRIM_CHECK_CUDA(cudaMemcpyToSymbol(c_asym_a0, a0, sizeof(a0)));
     GRIM_CHECK_CUDA(cudaMemcpyToSymbol(c_asym_a1, a1, sizeof(a1)));
-    double g0[GAL_ASYM64_TERMS], g1[GAL_ASYM64_TERMS];
-    g0[0] = g1[0] = 1.0;
-    for (int kk = 1; kk < GAL_ASYM64_TERMS; ++kk) {
-        const double odd = (2.0 * kk - 1.0) * (2.0 * kk - 1.0);
-        g0[kk] = g0[kk - 1] * (0.0 - odd) / (8.0 * kk);
-        g1[kk] = g1[kk - 1] * (4.0 - odd) / (8.0 * kk);
-    }
-    GRIM_CHECK_CUDA(cudaMemcpyToSymbol(c_gal_a0, g0, sizeof(g0)));
-    GRIM_CHECK_CUDA(cudaMemcpyToSymbol(c_gal_a1, g1, sizeof(g1)));
+    static const bool hankel_ready = (hankel_tables(), true);  // computed once for every device
+    (void)hankel_ready;
+    GRIM_CHECK_CUDA(cudaMemcpyToSymbol(c_hankel, &h_hankel, sizeof(h_hankel)));
     g_tables_ready[device] = 1;
     return GRIM_OK;
 }
@@ -415,13 +409,27 @@ static int gal_fill_impl(grim_context *h, int pol, int ne, int n, const double *
         if (split) cudaStreamWaitEvent(caller, h->events[1], 0);
         return status;
     }
+    // one thread per pair fills the chip (two CTAs of 256 threads an SM) from about 72 upper
+    // tiles on; below, eight threads share a pair.  Four CTAs per tile even out the last wave.
     const int tiles = ceil_div(ne, GAL_TILE);
-    dim3 fg(tiles, tiles);
+    const bool shared_pairs = (int64_t)tiles * (tiles + 1) * 2 < 2 * h->sm_count;
+    const int per_pair = shared_pairs ? GAL_FAR_LANES : 1;
+    dim3 fg(tiles, tiles, GAL_TILE * GAL_TILE * per_pair / GAL_FAR_THREADS);
+    auto far = [&](auto kernel, PerDeviceOnce &attr) -> int {
+        if (attr.needed()) {
+            GRIM_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GAL_FAR_SMEM));
+            attr.mark();
+        }
+        kernel<<<fg, GAL_FAR_THREADS, GAL_FAR_SMEM, h->stream>>>(ne, elem, nodes, k, far_min_order, E);
+        return grim_launch_status(h, "k_gal_far", 0, 0);
+    };
+    static PerDeviceOnce far_attr[4];
     if (pol == GRIM_POL_TM)
-        k_gal_far<GRIM_POL_TM, C><<<fg, GAL_FAR_THREADS, 0, h->stream>>>(ne, elem, nodes, k, far_min_order, E);
+        status = shared_pairs ? far(k_gal_far<GRIM_POL_TM, C, GAL_FAR_LANES>, far_attr[0])
+                              : far(k_gal_far<GRIM_POL_TM, C, 1>, far_attr[1]);
     else
-        k_gal_far<GRIM_POL_TE, C><<<fg, GAL_FAR_THREADS, 0, h->stream>>>(ne, elem, nodes, k, far_min_order, E);
-    status = grim_launch_status(h, "k_gal_far", 0, 0);
+        status = shared_pairs ? far(k_gal_far<GRIM_POL_TE, C, GAL_FAR_LANES>, far_attr[2])
+                              : far(k_gal_far<GRIM_POL_TE, C, 1>, far_attr[3]);
     if (split) GRIM_CHECK_CUDA(cudaStreamWaitEvent(caller, h->events[1], 0));
     GRIM_TRY(status);
     if (pol == GRIM_POL_TM)

@@ -1,0 +1,68 @@
+"""Far pairs of the linear-Galerkin fill against plain quadrature with SciPy's Bessel functions.
+
+Sizes sit at the edges of the 32-element tiles and on both sides of the switch between eight
+threads and one thread per pair; the wavenumbers reach every interval of the Hankel
+evaluation (x = 3, 4.5, 8, 25, 80) on one ring.  The tile orders hold a block within 1e-12 of
+a converged rule, so the matrices agree to 1e-12 of their largest entry."""
+import numpy as np
+import pytest
+from scipy import special
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip('torch')
+
+
+def _ring(count):
+    rng = np.random.default_rng(count)
+    theta = -2.0 * np.pi * (np.arange(count) + 0.2 * rng.uniform(-1, 1, count)) / count
+    return np.stack([np.cos(theta), 0.8 * np.sin(theta)], axis=1)
+
+
+def _far_entries(drawn, k, pol, rows, cols):
+    """Node entries (rows, cols) whose four element pairs are all far, by a 12-point rule."""
+    n = len(drawn)
+    a = drawn[(-np.arange(n)) % n]
+    b = np.roll(a, -1, axis=0)
+    length = np.hypot(*(b - a).T)
+    nrm = np.stack([-(b - a)[:, 1], (b - a)[:, 0]], axis=1) / length[:, None]
+    x, w = np.polynomial.legendre.leggauss(12)
+    x, w = 0.5 * (x + 1.0), 0.5 * w
+    hat = np.stack([1.0 - x, x])
+    out = np.zeros(len(rows), complex)
+    for eo, ao in ((rows, 0), ((rows - 1) % n, 1)):
+        for es, bs in ((cols, 0), ((cols - 1) % n, 1)):
+            po = a[eo][:, None, :] + x[None, :, None] * (b - a)[eo][:, None, :]
+            ps = a[es][:, None, :] + x[None, :, None] * (b - a)[es][:, None, :]
+            r = po[:, :, None, :] - ps[:, None, :, :]
+            d = np.hypot(r[..., 0], r[..., 1])
+            g = 0.25 * (special.y0(k * d) + 1j * special.j0(k * d))
+            h = 0.25 * k * (special.y1(k * d) + 1j * special.j1(k * d))
+            ll = length[eo] * length[es]
+            wt = np.einsum('p,q->pq', w * hat[ao], w * hat[bs])
+            s = ll * np.einsum('epq,pq->e', g, wt)
+            if pol == 'TM':
+                out += s + ll * np.einsum('epq,pq->e', h * np.einsum('epqx,ex->epq', r, nrm[es]) / d, wt) / (1j * k)
+            else:
+                kp = -ll * np.einsum('epq,pq->e', h * np.einsum('epqx,ex->epq', r, nrm[eo]) / d, wt)
+                total = np.einsum('epq,pq->e', g, np.einsum('p,q->pq', w, w))
+                sign = 1.0 if ao == bs else -1.0
+                hyper = -k * k * np.einsum('ex,ex->e', nrm[eo], nrm[es]) * s + sign * total
+                out += kp - hyper / (1j * k)
+    return out
+
+
+@pytest.mark.parametrize('n', [33, 64, 351, 352, 353, 385])
+@pytest.mark.parametrize('kl', [0.1, 0.6, 1.4])
+@pytest.mark.parametrize('pol', ['TM', 'TE'])
+def test_far_entries_equal_plain_quadrature(n, kl, pol):
+    from grim_20261007_b200.device import to_host_matrix
+    from grim_20261007_b200.twod.galerkin import GalerkinBody
+    drawn = _ring(n)
+    k = kl * n / 5.6
+    z = to_host_matrix(GalerkinBody([drawn]).fill_matrix(k, pol))
+    rng = np.random.default_rng(1)
+    rows = np.concatenate([rng.integers(0, n, 1500), np.repeat([0, 31, 32, n - 1], 40)])
+    gap = np.concatenate([rng.integers(8, n - 7, 1500), np.tile(np.linspace(8, n - 8, 40).astype(int), 4)])
+    cols = (rows + gap) % n
+    ref = _far_entries(drawn, k, pol, rows, cols)
+    assert np.max(np.abs(z[rows, cols] - ref)) <= 1e-12 * np.max(np.abs(z))
