@@ -812,18 +812,8 @@ static int gepp_rows_target(size_t csize) {
     return 128;
 }
 
-// Register-resident panel rows (k_panel_gepp_reg) for panels of at most 16 x GEPPR_ROWS rows;
-// GRIM_GEPP_REG=0 keeps every panel on the shared-memory kernel.
-static bool gepp_reg_enabled() {
-    static const bool on = [] {
-        const char *e = getenv("GRIM_GEPP_REG");
-        return !(e && atoi(e) == 0);
-    }();
-    return on;
-}
-
-// Loop-resident partial-pivoting panel (k_panel_gepp_loop) for panels of at most
-// 16 x GEPPL_ROWS rows; GRIM_GEPP_LOOP=0 keeps them on the unrolled register kernel.
+// Loop-resident partial-pivoting panel (k_panel_gepp_loop) for the panels whose rows fit the
+// registers of one cluster; GRIM_GEPP_LOOP=0 keeps every panel on the shared-memory kernel.
 static bool gepp_loop_enabled() {
     static const bool on = [] {
         const char *e = getenv("GRIM_GEPP_LOOP");
@@ -832,16 +822,33 @@ static bool gepp_loop_enabled() {
     return on;
 }
 
-// GRIM_GEPP_PUSH=1: candidate rows pushed into every CTA before the cluster barrier
-// (k_panel_gepp_loop PUSH).  Off by default: measured on the 2048-row panels it takes 132 us
-// against 119 us for reading only the winner's row through distributed shared memory after
-// the barrier (the pushes move 16 rows per CTA per column where the read moves one).
-static bool gepp_push_enabled() {
-    static const bool on = [] {
-        const char *e = getenv("GRIM_GEPP_PUSH");
-        return e && atoi(e) == 1;
-    }();
-    return on;
+// One launch of k_panel_gepp_loop: m panel rows on cs CTAs of THREADS / 2 row slots.
+template <typename C, int THREADS, bool SOLO>
+static int gepp_loop_launch(grim_context *h, int n, C *A, int64_t lda, int j, int nbj, int cs, int *ipiv, int *d_info,
+                            int *swapped, int *moves, PanelPack pk) {
+    const int m = n - j;
+    const size_t smem = (size_t)NB * (THREADS / 2) * sizeof(C);
+    auto kern = k_panel_gepp_loop<C, THREADS, SOLO>;
+    static PerDeviceOnce attr;
+    if (attr.needed()) {
+        GRIM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GRIM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr.mark();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(THREADS + GEPPL_HELPER);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute la[1];
+    la[0].id = cudaLaunchAttributeClusterDimension;
+    la[0].val.clusterDim.x = cs;
+    la[0].val.clusterDim.y = 1;
+    la[0].val.clusterDim.z = 1;
+    cfg.attrs = la;
+    cfg.numAttrs = 1;
+    GRIM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, n, A, lda, j, nbj, ceil_div(m, cs), ipiv, d_info, swapped, moves, pk));
+    return grim_launch_status(h, kname("k_panel_gepp_loop", sizeof(C)), 8.0 * m * nbj * nbj / 2.0, 0);
 }
 
 // Partial-pivoting factorization of the panel (j, nbj) of A on one thread-block cluster.
@@ -849,61 +856,22 @@ template <typename C>
 static int gepp_launch(grim_context *h, int n, C *A, int64_t lda, int j, int nbj, int *ipiv, int *d_info,
                        int *swapped, int *moves, PanelPack pk) {
     const int m = n - j;
-    if (gepp_loop_enabled() && m <= 16 * GEPPL_ROWS) {
-        const int cs = std::max(1, ceil_div(m, GEPPL_ROWS));
-        const int rpc = ceil_div(m, cs);
-        const bool push = gepp_push_enabled();
-        const size_t smem = ((size_t)NB * GEPPL_ROWS + (push ? (size_t)2 * 16 * 2 * NB : 0)) * sizeof(C);
-        auto kern = push ? k_panel_gepp_loop<C, true> : k_panel_gepp_loop<C, false>;
-        static PerDeviceOnce attr_loop;
-        if (attr_loop.needed()) {
-            for (auto kf : {k_panel_gepp_loop<C, true>, k_panel_gepp_loop<C, false>}) {
-                const size_t sm = ((size_t)NB * GEPPL_ROWS + (size_t)2 * 16 * 2 * NB) * sizeof(C);
-                GRIM_CHECK_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-                GRIM_CHECK_CUDA(cudaFuncSetAttribute(kf, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            }
-            attr_loop.mark();
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(GEPPL_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = h->stream;
-        cudaLaunchAttribute la[1];
-        la[0].id = cudaLaunchAttributeClusterDimension;
-        la[0].val.clusterDim.x = cs;
-        la[0].val.clusterDim.y = 1;
-        la[0].val.clusterDim.z = 1;
-        cfg.attrs = la;
-        cfg.numAttrs = 1;
-        GRIM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, n, A, lda, j, nbj, rpc, ipiv, d_info, swapped, moves, pk));
-        return grim_launch_status(h, kname("k_panel_gepp_loop", sizeof(C)), 8.0 * m * nbj * nbj / 2.0, 0);
+    constexpr int rows = GEPPL_THREADS / 2;
+    if (gepp_loop_enabled() && m <= rows)
+        return gepp_loop_launch<C, GEPPL_THREADS, true>(h, n, A, lda, j, nbj, 1, ipiv, d_info, swapped, moves, pk);
+    if (gepp_loop_enabled() && m <= 16 * rows) {
+        // 64 rows per CTA on up to 8 CTAs (the update of 128 rows outlasts the barrier it hides
+        // behind: m = 333 complex128 116 us a panel on 6 CTAs, 122 us on 3), then 128 (more CTAs
+        // make the barrier dearer: m = 1024 122 us on 8, 124 us on 16)
+        const int cs = std::max(ceil_div(m, rows), std::min(8, ceil_div(m, rows / 2)));
+        return gepp_loop_launch<C, GEPPL_THREADS, false>(h, n, A, lda, j, nbj, cs, ipiv, d_info, swapped, moves, pk);
     }
-    if (gepp_reg_enabled() && m <= 16 * GEPPR_ROWS) {
-        // rows in registers: the fewest CTAs of at most GEPPR_ROWS rows each
-        const int cs = std::max(1, ceil_div(m, GEPPR_ROWS));
-        const int rpc = ceil_div(m, cs);
-        static PerDeviceOnce attr_reg;
-        if (attr_reg.needed()) {
-            GRIM_CHECK_CUDA(
-                cudaFuncSetAttribute(k_panel_gepp_reg<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            attr_reg.mark();
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(GEPP_THREADS);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = h->stream;
-        cudaLaunchAttribute la[1];
-        la[0].id = cudaLaunchAttributeClusterDimension;
-        la[0].val.clusterDim.x = cs;
-        la[0].val.clusterDim.y = 1;
-        la[0].val.clusterDim.z = 1;
-        cfg.attrs = la;
-        cfg.numAttrs = 1;
-        GRIM_CHECK_CUDA(cudaLaunchKernelEx(&cfg, k_panel_gepp_reg<C>, n, A, lda, j, nbj, rpc, ipiv, d_info, swapped,
-                                           moves, pk));
-        return grim_launch_status(h, kname("k_panel_gepp_reg", sizeof(C)), 8.0 * m * nbj * nbj / 2.0, 0);
+    if constexpr (sizeof(C) == sizeof(float2)) {
+        // complex64 rows fit twice (m = 4096: 120 us a panel, 275 us with rows in shared memory)
+        constexpr int wide = GEPPL_THREADS_WIDE / 2;
+        if (gepp_loop_enabled() && m <= 16 * wide)
+            return gepp_loop_launch<C, GEPPL_THREADS_WIDE, false>(h, n, A, lda, j, nbj, ceil_div(m, wide), ipiv, d_info,
+                                                                  swapped, moves, pk);
     }
     const int target = gepp_rows_target(sizeof(C));
     int cs = 1;
