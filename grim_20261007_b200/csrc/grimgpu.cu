@@ -20,6 +20,7 @@
 #include "tc_gemm.cuh"
 #include "ozaki.cuh"
 #include "dmma.cuh"
+#include "trsolve.cuh"
 #include "grouped.cuh"
 #include "farblock.cuh"
 #include "galerkin.cuh"
@@ -1189,12 +1190,39 @@ static int rhs_interchanges(grim_context *h, int n, int nrhs, C *B, int64_t ldb,
     return GRIM_OK;
 }
 
+// Strip solves (k_trsolve_strip): a strip's time grows with n^2 on its one SM, the blocked
+// solve's with n (launches of 64-row blocks) until its GEMMs fill the chip.  One column meets
+// it at n = 2048 (1.87 ms either way), 181 columns at n = 3000 (4.0 ms); from 64 strips on the
+// strips fill the chip themselves (n = 4096, 720 columns 7.2 against 9.5 ms).
+static bool trsolve_wanted(int n, int nrhs) {
+    return tc_enabled() && (n <= 2048 || (n <= 3000 && nrhs >= 181) || nrhs >= 512);
+}
+
+template <bool UPPER>
+static int trsolve_strip(grim_context *h, int n, int nrhs, const double2 *LU, int64_t lda, double2 *B, int64_t ldb) {
+    static PerDeviceOnce attr;
+    if (attr.needed()) {
+        GRIM_CHECK_CUDA(
+            cudaFuncSetAttribute(k_trsolve_strip<UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRS_SMEM));
+        attr.mark();
+    }
+    k_trsolve_strip<UPPER><<<ceil_div(nrhs, TRS_COLS), TRS_THREADS, TRS_SMEM, h->stream>>>(n, nrhs, LU, lda, B, ldb);
+    GRIM_CHECK_LAUNCH_W(h, "k_trsolve_strip", 4.0 * n * n * nrhs, 16.0 * (0.5 * n * n + 2.0 * n * nrhs));
+    return GRIM_OK;
+}
+
 template <typename C>
 static int getrs_apply(grim_context *h, int n, int nrhs, const C *LU, int64_t lda, const int *ipiv, const int *ident,
                        C *B, int64_t ldb) {
     const int npan = ceil_div(n, NB);
     const size_t tri = (size_t)(NB * NBP + NB) * sizeof(C);
     GRIM_TRY(rhs_interchanges<C>(h, n, nrhs, B, ldb, ipiv, ident));
+    if constexpr (sizeof(C) == sizeof(double2)) {
+        if (trsolve_wanted(n, nrhs)) {
+            GRIM_TRY((trsolve_strip<false>(h, n, nrhs, LU, lda, B, ldb)));
+            return trsolve_strip<true>(h, n, nrhs, LU, lda, B, ldb);
+        }
+    }
     const int ctiles = ceil_div(nrhs, TRSM_COLS);
     for (int p = 0; p < npan; ++p) {
         const int j = p * NB, nbj = std::min(NB, n - j);

@@ -1,0 +1,180 @@
+// Triangular solves of complex128 getrs, one launch per triangle.
+//
+// The right-hand-side columns are independent, so a CTA takes a strip of eight of them (the
+// width of an FP64 tensor-core tile) through the whole substitution: no launch, no barrier
+// between CTAs per 64-row block.  (64-row blocks solved by one launch and applied by a
+// rank-64 GEMM by another spend 12 us and 25-50 us a block on launches, prologues and
+// partly filled waves: N = 2048, 720 columns 2.1 ms a triangle.)
+// Per 64-row block i, with X the solved rows of the strip:
+//   1. W = B_i - T_i X over every solved row (mma.sync m8n8k4 .f64): sixteen warps, each eight
+//      rows by every other group of four k-steps (eight warps left half the tensor pipe idle:
+//      two a scheduler do not cover the instructions between the MMAs).  Fragments come
+//      straight from L2 -- eight consecutive rows of a column are one 128-byte line, read once
+//      per strip -- two groups ahead; the solved rows, read by eight warps, from L1;
+//      meanwhile the diagonal block arrives in shared memory with cp.async;
+//   2. the 64-row substitution, one warp per column, two rows per lane;
+//   3. X_i to global memory, where step 1 of the next block reads it.
+// Bound by the FP64 tensor pipe of the SMs that have a strip (8 n^2 x 8 / 2 flops a strip and
+// triangle) and the substitution chain (about 4 us a block).  getrs, both triangles with the
+// interchanges, blocked launches before -> strips: N = 400, 722 columns 0.53 -> 0.18 ms;
+// N = 1024, 361 1.30 -> 0.61 ms; N = 2048, 720 3.40 -> 1.99 ms; N = 4096, 720 9.5 -> 7.2 ms.
+#pragma once
+#include "dmma.cuh"
+#include "lu.cuh"
+
+#define TRS_COLS 8
+#define TRS_THREADS 512
+#define TRS_GROUP 4   // k-steps (of four columns of T) per prefetched group
+#define TRS_DEPTH 1   // groups in flight ahead of the one multiplied (odd: two B buffers alternate)
+#define TRS_LDT (NB + 1)
+#define TRS_SMEM ((size_t)(NB * TRS_LDT + 2 * TRS_COLS * TRS_LDT + NB) * sizeof(double2))
+
+// A read-once element of the factor: not kept in L1 (the solved rows, read by all eight warps,
+// are).
+__device__ __forceinline__ double2 trs_stream(const double2 *p) {
+    double2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
+template <bool UPPER>
+__global__ void __launch_bounds__(TRS_THREADS, 1)
+k_trsolve_strip(int n, int nrhs, const double2 *__restrict__ LU, int64_t lda, double2 *B, int64_t ldb) {
+    extern __shared__ __align__(16) unsigned char trs_smem[];
+    double2 *T = reinterpret_cast<double2 *>(trs_smem);  // [column][TRS_LDT] diagonal block
+    double2 *W = T + NB * TRS_LDT;                        // [strip column][TRS_LDT], and the odd groups' sums
+    double2 *rd = W + 2 * TRS_COLS * TRS_LDT;                 // reciprocals of the diagonal
+    const int t = threadIdx.x, warp = (t >> 5) & 7, odd = t >> 8, lane = t & 31, g = lane >> 2, q = lane & 3;
+    const int c0 = blockIdx.x * TRS_COLS, nblk = (n + NB - 1) / NB;
+    const double2 *bcol = B + (int64_t)min(c0 + g, nrhs - 1) * ldb;
+    for (int s = 0; s < nblk; ++s) {
+        const int i = UPPER ? nblk - 1 - s : s, j = i * NB, nbj = min(NB, n - j);
+        for (int e = t; e < NB * NB; e += TRS_THREADS) {
+            const int r = e % NB, c = e / NB;
+            const bool ok = r < nbj && c < nbj && (UPPER ? r <= c : r > c);
+            dm_cp16(T + c * TRS_LDT + r, ok ? (const void *)(LU + (int64_t)(j + c) * lda + j + r) : (const void *)LU, ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        // solved rows [k0, k1), oldest first: forward from row 0, backward from row n - 1 (a
+        // last partial group there, its missing rows skipped; every other group is whole)
+        const int k0 = UPPER ? j + nbj : 0, k1 = UPPER ? n : j;
+        const int row = j + 8 * warp + g;
+        const bool row_ok = row < n;
+        // rows past n and columns past nrhs repeat the last one: their sums are not stored
+        const double2 *ap = LU + (row_ok ? row : n - 1) + (int64_t)(k0 + q) * lda, *bp = bcol + k0 + q;
+        const int ngrp = (k1 - k0 + 4 * TRS_GROUP - 1) / (4 * TRS_GROUP), mine = (ngrp + 1 - odd) / 2;
+        double re[TRS_GROUP][2] = {}, im[TRS_GROUP][2] = {};
+        double2 a[TRS_DEPTH + 1][TRS_GROUP], b[2][TRS_GROUP];
+        auto load_a = [&](double2(&v)[TRS_GROUP], int grp) {
+            if (grp >= mine) return;
+            const int off = 4 * TRS_GROUP * (UPPER ? ngrp - 1 - 2 * grp - odd : 2 * grp + odd);
+            const double2 *p = ap + (int64_t)off * lda;
+            const bool whole = k0 + off + 4 * TRS_GROUP <= k1;
+#pragma unroll
+            for (int u = 0; u < TRS_GROUP; ++u) {
+                if (whole || k0 + off + q + 4 * u < k1) v[u] = trs_stream(p + (int64_t)(4 * u) * lda);
+                else v[u] = czero<double2>();
+            }
+        };
+        auto load_b = [&](double2(&v)[TRS_GROUP], int grp) {
+            if (grp >= mine) return;
+            const int off = 4 * TRS_GROUP * (UPPER ? ngrp - 1 - 2 * grp - odd : 2 * grp + odd);
+            const bool whole = k0 + off + 4 * TRS_GROUP <= k1;
+#pragma unroll
+            for (int u = 0; u < TRS_GROUP; ++u) {
+                if (whole || k0 + off + q + 4 * u < k1) v[u] = bp[off + 4 * u];
+                else v[u] = czero<double2>();
+            }
+        };
+        // the group's k-steps side by side, each its own accumulators
+        auto mma = [&](const double2(&x)[TRS_GROUP], const double2(&y)[TRS_GROUP]) {
+#pragma unroll
+            for (int u = 0; u < TRS_GROUP; ++u) {
+                dmma(re[u][0], re[u][1], x[u].x, y[u].x);
+                dmma(im[u][0], im[u][1], x[u].x, y[u].y);
+            }
+#pragma unroll
+            for (int u = 0; u < TRS_GROUP; ++u) {
+                dmma(re[u][0], re[u][1], -x[u].y, y[u].y);
+                dmma(im[u][0], im[u][1], x[u].y, y[u].x);
+            }
+        };
+#pragma unroll
+        for (int v = 0; v < TRS_DEPTH; ++v) load_a(a[v], v);
+        load_b(b[0], 0);
+        for (int grp = 0; grp < mine; grp += TRS_DEPTH + 1) {
+#pragma unroll
+            for (int v = 0; v < TRS_DEPTH + 1; ++v) {
+                if (grp + v >= mine) break;
+                load_a(a[(v + TRS_DEPTH) % (TRS_DEPTH + 1)], grp + v + TRS_DEPTH);
+                load_b(b[(v + 1) % 2], grp + v + 1);
+                mma(a[v], b[v % 2]);
+            }
+        }
+#pragma unroll
+        for (int u = 1; u < TRS_GROUP; ++u)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                re[0][e] += re[u][e];
+                im[0][e] += im[u][e];
+            }
+        // lane holds row 8 warp + g, strip columns 2 q, 2 q + 1
+        if (odd) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                W[(TRS_COLS + 2 * q + e) * TRS_LDT + 8 * warp + g] = make_double2(re[0][e], im[0][e]);
+        }
+        __syncthreads();
+        if (!odd) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = 2 * q + e;
+                double2 v = czero<double2>();
+                if (row_ok && c0 + c < nrhs) v = B[(int64_t)(c0 + c) * ldb + row];
+                const double2 w = W[(TRS_COLS + c) * TRS_LDT + 8 * warp + g];
+                W[c * TRS_LDT + 8 * warp + g] = make_double2(v.x - (re[0][e] + w.x), v.y - (im[0][e] + w.y));
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (UPPER && t < NB) rd[t] = t < nbj ? crecip(T[t * TRS_LDT + t]) : czero<double2>();
+        if (UPPER) __syncthreads();
+        // one column per warp (the first eight); rows at and past nbj hold zeros and are left alone
+        if (!odd) {
+            double2 x0 = W[warp * TRS_LDT + lane], x1 = W[warp * TRS_LDT + lane + 32];
+            if (!UPPER) {
+#pragma unroll 8
+                for (int k = 0; k < 32; ++k) {
+                    const double2 xk = shfl_c(x0, k);
+                    if (lane > k) cfms(x0, T[k * TRS_LDT + lane], xk);
+                    cfms(x1, T[k * TRS_LDT + lane + 32], xk);
+                }
+#pragma unroll 8
+                for (int k = 32; k < NB; ++k) {
+                    const double2 xk = shfl_c(x1, k - 32);
+                    if (lane > k - 32) cfms(x1, T[k * TRS_LDT + lane + 32], xk);
+                }
+            } else {
+#pragma unroll 8
+                for (int k = NB - 1; k >= 32; --k) {
+                    if (lane == k - 32) x1 = cmul(x1, rd[k]);
+                    const double2 xk = shfl_c(x1, k - 32);
+                    if (lane < k - 32) cfms(x1, T[k * TRS_LDT + lane + 32], xk);
+                    cfms(x0, T[k * TRS_LDT + lane], xk);
+                }
+#pragma unroll 8
+                for (int k = 31; k >= 0; --k) {
+                    if (lane == k) x0 = cmul(x0, rd[k]);
+                    const double2 xk = shfl_c(x0, k);
+                    if (lane < k) cfms(x0, T[k * TRS_LDT + lane], xk);
+                }
+            }
+            if (c0 + warp < nrhs) {
+                double2 *out = B + (int64_t)(c0 + warp) * ldb + j;
+                if (lane < nbj) out[lane] = x0;
+                if (lane + 32 < nbj) out[lane + 32] = x1;
+            }
+        }
+        __syncthreads();  // X_i in place, T and W free
+    }
+}

@@ -1,0 +1,59 @@
+"""FP64 getrs in strips of eight columns against SciPy's lu_solve, at the edges of the 64-row
+blocks and of the strips, with padded leading dimensions, and at a zero or infinite entry."""
+import ctypes
+
+import numpy as np
+import pytest
+import scipy.linalg as sla
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip('torch')
+
+
+def _getrs(lu, piv, b, lda, ldb):
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.device import context, ptr
+    ctx = context()
+    n, nrhs = b.shape
+    a = torch.zeros((n, lda), dtype=torch.complex128)
+    a[:, :n] = torch.from_numpy(np.ascontiguousarray(lu.T))
+    x = torch.full((nrhs, ldb), 7.0 - 3.0j, dtype=torch.complex128)
+    x[:, :n] = torch.from_numpy(np.ascontiguousarray(b.T))
+    a, x = a.cuda(), x.cuda()
+    ip = torch.from_numpy((piv + 1).astype(np.int32)).cuda()
+    _lib.check(ctx.lib.grim_zgetrs(ctx.h, n, nrhs, ptr(a), lda, ptr(ip), ptr(x), ldb))
+    out = x.cpu().numpy()
+    assert np.all(out[:, n:] == 7.0 - 3.0j)  # the padding rows stay as they were
+    return out[:, :n].T
+
+
+@pytest.mark.parametrize('n', [1, 8, 63, 64, 65, 129, 200, 321])
+@pytest.mark.parametrize('nrhs', [1, 7, 8, 9, 33])
+def test_getrs_strips_equal_scipy(n, nrhs):
+    rng = np.random.default_rng(1000 * n + nrhs)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    lu, piv = sla.lu_factor(a)
+    x = _getrs(lu, piv, b, n + 3, n + 5)
+    ref = sla.lu_solve((lu, piv), b)
+    # normwise backward error of a substitution: a few n eps of |A| |x|
+    res = np.max(np.abs(a @ x - b), axis=0)
+    den = np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x), axis=0)
+    assert np.max(res / den) < 1e-14
+    assert np.max(np.abs(x - ref)) <= 1e-12 * np.linalg.cond(a) * np.max(np.abs(ref))
+
+
+def test_getrs_strips_keep_columns_apart():
+    """An infinite right-hand side entry stays in its own column."""
+    n = 130
+    rng = np.random.default_rng(5)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    b = rng.standard_normal((n, 11)) + 1j * rng.standard_normal((n, 11))
+    lu, piv = sla.lu_factor(a)
+    clean = _getrs(lu, piv, b, n, n)
+    b2 = b.copy()
+    b2[40, 3] = np.inf
+    x = _getrs(lu, piv, b2, n, n)
+    keep = [c for c in range(11) if c != 3]
+    assert np.array_equal(x[:, keep], clean[:, keep])
+    assert not np.all(np.isfinite(x[:, 3]))
