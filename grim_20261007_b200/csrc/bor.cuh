@@ -12,10 +12,20 @@
 //            momk[((e * ne + f) * (mmax + 2) + n) * 16 + 4 uv + 2 a + c], complex128.
 //   The element pairs follow the reference's routing (bor/solver.py:1520-1580): far pairs
 //   take 3 x 3 Gauss points and the uniform trapezoid rule in xi (k_bor_far, one CTA per
-//   pair); near pairs take the host's point list -- graded cells for self / adjacent pairs
-//   (bor/solver.py:718-806), a 12 x 12 Gauss rule for the others (:843) -- and a composite
-//   rule on xi in [0, pi] using each integrand's parity (k_bor_near over work items of at
-//   most BOR_NEAR_CHUNK point pairs, then k_bor_near_reduce in a fixed order).
+//   pair, three warps of three point pairs); near pairs take the host's point list -- graded cells for
+//   self / adjacent pairs (bor/solver.py:718-806), a 12 x 12 Gauss rule for the others (:843)
+//   -- and a composite rule on xi in [0, pi] using each integrand's parity (k_bor_near over
+//   work items of at most BOR_NEAR_CHUNK point pairs, one warp per point pair, then
+//   k_bor_near_reduce in a fixed order).
+//
+// Both kernels are bound by the FP64 pipe: per sample about 70 operations for the kernel
+// values and, per order n, ten sums (G and the even brackets against cos n xi, the odd ones
+// against sin n xi, re and im) plus four operations to turn e^{j n xi}.  A lane keeps the sums
+// of MB orders, so that each value it reads from shared memory feeds MB of them (one order
+// per thread: five 16-byte loads per ten sums, shared-memory bound at 32 % of the FP64 pipe).
+// The far rule's samples are folded twice (xi -> -xi by parity in xi, xi -> pi - xi by parity
+// in n), which leaves a quarter of the sums and half of the kernel values.  400-segment ogive,
+// 42 orders, CFIE: far 30.9 -> 13.2 ms, near 41.4 -> 13.4 ms (near: 48 % of the FP64 pipe).
 // Stage 2  k_bor_assemble: the reduced mode-m matrix alpha C EFIE + (1 - alpha) eta0
 //   ((1/2) M - K), C = j k eta 2 pi, from the moments of the <= 4 element pairs touching
 //   each node pair, with the pole treatment (inactive pole phi components, |m| = 1 pole t
@@ -28,6 +38,7 @@
 // farfield_vv_hh_batch), :4285-4301 (CFIE), bor/kernels.py:896,996 (MFIE brackets).
 #pragma once
 #include "common.cuh"
+#include "hankel64.cuh"
 
 #define BOR_FAR_ORDER 3
 #define BOR_MAX_MODES 128
@@ -35,11 +46,14 @@
 #define BOR_SLOTS 20
 #define BOR_KSLOTS 16
 #define BOR_ALL_SLOTS (BOR_SLOTS + BOR_KSLOTS)
-#define BOR_THREADS 256
-#define BOR_FAR_CHUNK 256   // far-pair xi samples staged per pass
+#define BOR_CHUNK 32        // samples a warp stages per pass (one per lane)
+#define BOR_FAR_WARPS 3        // warps of a far CTA, three of the nine point pairs each
+#define BOR_FAR_PAIRS (BOR_FAR_ORDER * BOR_FAR_ORDER)
+#define BOR_NEAR_WARPS 8
 #define BOR_NEAR_CHUNK 64   // point pairs per near work item
 #define BOR_XI_CORE 20      // Gauss points of the near rule's sinh core
-#define BOR_XI_PANEL 16     // Gauss points per panel of the near rule
+#define BOR_XI_PANEL 16     // Gauss points per doubling panel of the near rule
+#define BOR_XI_WIDE 32      // Gauss points per panel of its uniform part
 
 struct BorPt {
     double rho, z, w, T0, T1, D0, D1, tr, tz;
@@ -76,58 +90,69 @@ __device__ __forceinline__ void gl_node(int q, int i, double &x, double &w) {
     w = c_gl_w[q * (q - 1) / 2 + i];
 }
 
-// Geometry of one point pair shared by every xi sample.
+// Geometry of one point pair shared by every xi sample; the MFIE brackets as functions of
+// h = 1 - cos xi and sin xi: tt = tt0 + h tt1, tf = tf1 sin xi, ft = ft1 sin xi, ff = ff0 + h ff1
+// (cancellation-free forms).
 struct BorPair {
-    double k, rp, rq, dr, dz, d2, rr2;     // rr2 = 2 rho rho'
-    double A, N, X, D, trp, tzp, trq, tzq;  // MFIE bracket invariants
+    double k, d2, rr2;  // rr2 = 2 rho rho'
+    double tt0, tt1, tf1, ft1, ff0, ff1;
 };
 
 __device__ __forceinline__ BorPair bor_pair(double k, const BorPt &p, const BorPt &q) {
     BorPair s;
     s.k = k;
-    s.rp = p.rho;
-    s.rq = q.rho;
-    s.dr = p.rho - q.rho;
-    s.dz = p.z - q.z;
-    s.d2 = s.dr * s.dr + s.dz * s.dz;
+    const double dr = p.rho - q.rho, dz = p.z - q.z;
+    s.d2 = dr * dr + dz * dz;
     s.rr2 = 2.0 * p.rho * q.rho;
-    s.trp = p.tr;
-    s.tzp = p.tz;
-    s.trq = q.tr;
-    s.tzq = q.tz;
-    s.X = p.tr * q.tz - p.tz * q.tr;
-    s.D = p.tr * q.tr + p.tz * q.tz;
-    s.A = p.tr * s.dr + p.tz * s.dz;
-    s.N = -p.tz * s.dr + p.tr * s.dz;
+    const double X = p.tr * q.tz - p.tz * q.tr, D = p.tr * q.tr + p.tz * q.tz;
+    const double A = p.tr * dr + p.tz * dz, N = -p.tz * dr + p.tr * dz;
+    s.tt0 = A * X - D * N;
+    s.tt1 = A * p.tz * q.tr + p.tr * q.rho * X + D * p.tz * q.rho + p.tr * q.tr * N;
+    s.tf1 = -dz * (p.tr * p.tr + p.tz * p.tz);
+    s.ft1 = q.rho * X + q.tr * N;
+    s.ff0 = -N;
+    s.ff1 = N - p.tz * q.rho;
     return s;
 }
 
 // One xi sample times weight wt: the Green's function g and (MFIE) the four brackets
-// -p(R) [tt, tf, ft, ff] in the cancellation-free form (h = 1 - cos xi = 2 sin^2(xi/2)).
+// -p(R) [tt, tf, ft, ff], from sin(xi/2) and sin xi.  1/R from the hardware estimate and a
+// third-order correction, R corrected to half an ulp.
 template <bool MFIE>
 __device__ __forceinline__ void bor_sample(const BorPair &s, double shalf, double sx, double wt, double2 &g,
                                            double2 (&F)[4]) {
     const double h = 2.0 * shalf * shalf;
-    const double R = sqrt(s.d2 + s.rr2 * h);
+    const double R2 = fma(s.rr2, h, s.d2);
+    double ir;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(ir) : "d"(R2));
+    const double e = fma(-R2 * ir, ir, 1.0);
+    ir = fma(ir * e, fma(e, 0.375, 0.5), ir);
+    double R = R2 * ir;
+    R = fma(0.5 * ir, fma(-R, R, R2), R);
+    const double kr = s.k * R;
     double sk, ck;
-    sincos(s.k * R, &sk, &ck);
-    const double a = wt / (4.0 * GRIM_PI * R);
+    gh_sincos(kr, sk, ck);
+    const double a = wt * (1.0 / (4.0 * GRIM_PI)) * ir;
     g = make_double2(a * ck, -a * sk);
     if constexpr (MFIE) {
-        const double kr = s.k * R;
-        const double pre = a / (R * R);
+        const double pre = a * (ir * ir);
         // -(1 + j kR) e^{-jkR} / (4 pi R^3) times the weight
-        const double pr = -pre * (ck + kr * sk), pi = -pre * (kr * ck - sk);
-        const double tt = (s.A * s.X - s.D * s.N) +
-                          h * (s.A * s.tzp * s.trq + s.trp * s.rq * s.X + s.D * s.tzp * s.rq + s.trp * s.trq * s.N);
-        const double tf = -sx * s.dz * (s.trp * s.trp + s.tzp * s.tzp);
-        const double ft = sx * (s.rq * s.X + s.trq * s.N);
-        const double ff = -s.tzp * s.rq * h - s.N * (1.0 - h);
+        const double pr = -pre * fma(kr, sk, ck), pi = pre * fma(-kr, ck, sk);
+        const double tt = fma(h, s.tt1, s.tt0), tf = s.tf1 * sx, ft = s.ft1 * sx, ff = fma(h, s.ff1, s.ff0);
         F[0] = make_double2(pr * tt, pi * tt);
         F[1] = make_double2(pr * tf, pi * tf);
         F[2] = make_double2(pr * ft, pi * ft);
         F[3] = make_double2(pr * ff, pi * ff);
     }
+}
+
+// e^{2 pi j i / N}, 0 <= i < N: the quadrant exactly, then the polynomials.  One copy: k_bor_far
+// waited for instructions a third of the time with it (and two kernel samples) inlined.
+__device__ __noinline__ double2 bor_unit(int i, int N) {
+    const int q = (4 * i + (N >> 1)) / N, rem = 4 * i - q * N;
+    double sn, cs;
+    gh_sincos_quadrant(rem * (0.5 * GRIM_PI / N), q, sn, cs);
+    return make_double2(cs, sn);
 }
 
 // The 36 per-point-pair factors multiplying G_n (slots 0..19) or K^n_uv (slots 20..35).
@@ -146,142 +171,155 @@ __device__ __forceinline__ double bor_factor(const BorPt &p, const BorPt &q, int
     }
 }
 
-// Shared-memory layout of the moment kernels (sizes from the host: nm modes, nsl slots).
-//   acc[nm * nsl]   running moments of the CTA's element pair / work item
-//   red[S * nm * 5] per-group partial sums of G_n and K^n_uv
-//   fac[nsl]        the current point pair's factors
-//   sum[nm * 5]     G_n, K^n_uv of the current point pair
-template <bool MFIE>
-__device__ __forceinline__ void bor_fold_pair(int nm, int S, double2 *red, double2 *sum, const double *fac,
-                                              double2 *acc) {
-    constexpr int NV = MFIE ? 5 : 1, nsl = MFIE ? BOR_ALL_SLOTS : BOR_SLOTS;
-    const int t = threadIdx.x;
-    // reduce the groups in a fixed order
-    for (int i = t; i < nm * NV; i += blockDim.x) {
-        double2 v = make_double2(0.0, 0.0);
-        for (int gq = 0; gq < S; ++gq) {
-            const double2 r = red[gq * nm * NV + i];
-            v.x += r.x;
-            v.y += r.y;
-        }
-        sum[i] = v;
-    }
-    __syncthreads();
-    for (int i = t; i < nm * nsl; i += blockDim.x) {
-        const int n = i / nsl, slot = i - n * nsl;
-        double2 v;
-        if (slot < BOR_SLOTS) {
-            v = sum[n * NV];
-        } else {
-            const int uv = (slot - BOR_SLOTS) >> 2;
-            const double2 kv = sum[n * NV + 1 + uv];
-            // odd brackets: K = -j sum F sin(n xi)
-            v = (uv == 1 || uv == 2) ? make_double2(kv.y, -kv.x) : kv;
-        }
-        const double f = fac[slot];
-        acc[i].x += f * v.x;
-        acc[i].y += f * v.y;
-    }
-    __syncthreads();
+// Lanes of a warp over the orders n < nm: blocks of MB orders, G = 32 / blocks lanes sharing a
+// block (each every G-th sample).
+__host__ __device__ constexpr int bor_far_blocks(int nm, int mb) { return 2 * (((nm + 1) / 2 + mb - 1) / mb); }
+__host__ __device__ constexpr int bor_near_blocks(int nm, int mb) { return (nm + mb - 1) / mb; }
+// Orders per lane: three (two CTAs of registers an SM), four where three need over 32 lanes.
+__host__ __device__ constexpr int bor_mb(int nm) {
+    return bor_far_blocks(nm, 3) <= 32 && bor_near_blocks(nm, 3) <= 32 ? 3 : 4;
 }
 
-// grid = (ne, ne), BOR_THREADS threads; pairs with cls != 0 return at once.  Thread
-// (n = t % nm, grp = t / nm) sums mode n over the samples i = grp (mod S) of each point pair,
-// with e^{j n xi_i} carried by rotation and re-anchored exactly every 32 of them; the groups'
-// sums of each of the 9 point pairs are reduced in shared memory, and the 36 slot moments
-// are formed once at the end.
-// dynamic smem: samples [NV][BOR_FAR_CHUNK], red[S][nm][NV], sums[9][nm][NV], fac[9][nsl].
-template <bool MFIE>
-__global__ void __launch_bounds__(BOR_THREADS, 2)
+// The lanes' sums over the groups g = 1.. of their block, added in order; group 0 holds them.
+template <int COUNT>
+__device__ __forceinline__ void bor_sum_groups(double2 (&v)[COUNT], int block, int blocks, int groups) {
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) {
+        const double2 own = v[i];
+        for (int g = 1; g < groups; ++g) {
+            v[i].x += __shfl_sync(0xffffffffu, own.x, block + g * blocks);
+            v[i].y += __shfl_sync(0xffffffffu, own.y, block + g * blocks);
+        }
+    }
+}
+
+// grid = (ne, ne), BOR_FAR_WARPS warps, warp w the point pairs 3 w .. 3 w + 2 of the element
+// pair (nine warps leave 96 registers a thread, and the sums of MB orders spill); pairs with
+// cls != 0 return at once.  A lane keeps MB orders of one parity (n = par + 2 i), whose
+// folded samples are f(xi) +- f(pi - xi); e^{j n xi} is carried by rotation over G samples and
+// re-anchored exactly every second chunk.
+// dynamic smem: fold[warp][2 NV][BOR_CHUNK], sums[pair][nm][NV], fac[pair][nsl].
+template <bool MFIE, int MB>
+__global__ void __launch_bounds__(32 * BOR_FAR_WARPS, 4)
 k_bor_far(int ne, const double *__restrict__ nodes, const unsigned char *__restrict__ cls, double k, int mmax,
           int nxi_cap, double2 *__restrict__ mom, double2 *__restrict__ momk) {
     constexpr int NV = MFIE ? 5 : 1, nsl = MFIE ? BOR_ALL_SLOTS : BOR_SLOTS;
-    constexpr int NPP = BOR_FAR_ORDER * BOR_FAR_ORDER;
     const int e = blockIdx.x, f = blockIdx.y;
     if (cls[(int64_t)e * ne + f] != 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int nm = mmax + 2, S = BOR_THREADS / nm;
-    double2 *chunk = reinterpret_cast<double2 *>(smem_raw);  // [NV][BOR_FAR_CHUNK]
-    double2 *red = chunk + NV * BOR_FAR_CHUNK;                // [S][nm][NV]
-    double2 *sums = red + S * nm * NV;                         // [NPP][nm][NV]
-    double *fac = reinterpret_cast<double *>(sums + NPP * nm * NV);  // [NPP][nsl]
-    const int t = threadIdx.x, n = t % nm, grp = t / nm;
-    for (int pp = 0; pp < NPP; ++pp) {
-        const int ip = pp / BOR_FAR_ORDER, iq = pp % BOR_FAR_ORDER;
+    const int nm = mmax + 2, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double2 *fold = reinterpret_cast<double2 *>(smem_raw) + warp * 2 * NV * BOR_CHUNK;
+    double2 *sums = reinterpret_cast<double2 *>(smem_raw) + BOR_FAR_WARPS * 2 * NV * BOR_CHUNK;
+    double *fac = reinterpret_cast<double *>(sums + BOR_FAR_PAIRS * nm * NV);
+    const int blocks = bor_far_blocks(nm, MB), groups = 32 / blocks;
+    const int block = lane % blocks, grp = lane / blocks, par = block & 1, n0 = par + 2 * MB * (block >> 1);
+#pragma unroll 1
+    for (int pp = warp * (BOR_FAR_PAIRS / BOR_FAR_WARPS); pp < (warp + 1) * (BOR_FAR_PAIRS / BOR_FAR_WARPS); ++pp) {
         double xo, wo, xs, wsq;
-        gl_node(BOR_FAR_ORDER, ip, xo, wo);
-        gl_node(BOR_FAR_ORDER, iq, xs, wsq);
+        gl_node(BOR_FAR_ORDER, pp / BOR_FAR_ORDER, xo, wo);
+        gl_node(BOR_FAR_ORDER, pp % BOR_FAR_ORDER, xs, wsq);
         const BorPt p = bor_point(nodes, e, 0.5 * (xo + 1.0), 0.5 * wo);
         const BorPt q = bor_point(nodes, f, 0.5 * (xs + 1.0), 0.5 * wsq);
-        if (t < nsl) fac[pp * nsl + t] = bor_factor(p, q, t);
+        for (int s = lane; s < nsl; s += 32) fac[pp * nsl + s] = bor_factor(p, q, s);
         const BorPair pr = bor_pair(k, p, q);
         const int N = min(bor_nxi(k, p.rho, q.rho, sqrt(pr.d2), mmax), nxi_cap);
         const double dxi = 2.0 * GRIM_PI / N;
-        double2 sg = make_double2(0.0, 0.0), s1 = sg, s2 = sg, s3 = sg, s4 = sg;
-        // rotation by n S samples (n < 128, N <= 8192: 32-bit phase indices)
-        double rs, rc;
-        sincospi(2.0 * (double)((n * S) % N) / N, &rs, &rc);
-        for (int i0 = 0; i0 < N; i0 += BOR_FAR_CHUNK) {
-            const int cnt = min(BOR_FAR_CHUNK, N - i0);
-            __syncthreads();
-            for (int j = t; j < cnt; j += blockDim.x) {
-                const int i = i0 + j;
-                double sh, ch;
-                sincospi(i / (double)N, &sh, &ch);
-                double2 g, F[4];
-                bor_sample<MFIE>(pr, sh, 2.0 * sh * ch, dxi, g, F);
-                chunk[j] = g;
-                if constexpr (MFIE) {
+        double2 acc[MB][NV], z[MB], rot[MB];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) chunk[(1 + u) * BOR_FAR_CHUNK + j] = F[u];
+        for (int m = 0; m < MB; ++m) {
+            // e^{j n dxi}; its powers: the lane's first sample (grp) and its step (groups)
+            const double2 w = bor_unit((n0 + 2 * m) % N, N);
+            double2 pw = make_double2(1.0, 0.0);
+            z[m] = pw;
+#pragma unroll 1
+            for (int g = 0; g < groups; ++g) {
+                if (g == grp) z[m] = pw;
+                pw = cmul(pw, w);
+            }
+            rot[m] = pw;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[m][v] = make_double2(0.0, 0.0);
+        }
+        int i = grp < groups ? grp : 0x3fffffff;  // this lane's next folded sample
+        const double2 *set = fold + par * NV * BOR_CHUNK;
+        const int last = N / 4;
+        for (int i0 = 0; i0 <= last; i0 += BOR_CHUNK) {
+            // raw values at xi (side 0) and pi - xi (side 1) of the chunk's points: 2 cnt tasks (xi =
+            // pi/2 is its own partner), then the folds in place -- even n: the sum of the even
+            // functions and the difference of the odd ones; odd n: the other way round
+            const int cnt = min(BOR_CHUNK, last + 1 - i0);
+            __syncwarp();
+#pragma unroll 1
+            for (int task = lane; task < 2 * cnt; task += 32) {
+                const int side = task >= cnt, at = side ? task - cnt : task, is = i0 + at;
+                double2 val[5];
+                if (side && is == last) {
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) val[v] = make_double2(0.0, 0.0);
+                } else {
+                    const double2 u = bor_unit(side ? N / 2 - is : is, 2 * N);  // e^{j xi / 2}
+                    double2 F[4];
+                    bor_sample<MFIE>(pr, u.y, 2.0 * u.y * u.x, is == 0 ? dxi : 2.0 * dxi /* xi and -xi */, val[0], F);
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) val[1 + v] = F[v];
+                }
+#pragma unroll
+                for (int v = 0; v < NV; ++v) fold[(side * NV + v) * BOR_CHUNK + at] = val[v];
+            }
+            __syncwarp();
+            if (lane < cnt) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const bool odd = v == 2 || v == 3;
+                    const double2 x = fold[v * BOR_CHUNK + lane], y = fold[(NV + v) * BOR_CHUNK + lane];
+                    fold[v * BOR_CHUNK + lane] = odd ? csub(x, y) : cadd(x, y);
+                    fold[(NV + v) * BOR_CHUNK + lane] = odd ? cadd(x, y) : csub(x, y);
                 }
             }
-            __syncthreads();
-            if (grp < S) {
-                // samples i = grp (mod S); e^{j n xi_i} anchored exactly every 32 of them
-                int j = (grp - i0 % S + S) % S;
-                while (j < cnt) {
-                    double zs, zc;
-                    sincospi(2.0 * (double)((n * (i0 + j)) % N) / N, &zs, &zc);
-                    double2 z = make_double2(zc, zs);
-                    const int jend = min(cnt, j + 32 * S);
-#pragma unroll(MFIE ? 2 : 4)
-                    for (; j < jend; j += S) {
-                        const double2 v = chunk[j];
-                        sg.x += v.x * z.x;
-                        sg.y += v.y * z.x;
-                        if constexpr (MFIE) {
-                            const double2 f0 = chunk[BOR_FAR_CHUNK + j], f1 = chunk[2 * BOR_FAR_CHUNK + j];
-                            const double2 f2 = chunk[3 * BOR_FAR_CHUNK + j], f3 = chunk[4 * BOR_FAR_CHUNK + j];
-                            s1.x += f0.x * z.x; s1.y += f0.y * z.x;
-                            s2.x += f1.x * z.y; s2.y += f1.y * z.y;
-                            s3.x += f2.x * z.y; s3.y += f2.y * z.y;
-                            s4.x += f3.x * z.x; s4.y += f3.y * z.x;
-                        }
-                        z = make_double2(z.x * rc - z.y * rs, z.x * rs + z.y * rc);
+            __syncwarp();
+            const int iend = min(i0 + BOR_CHUNK, last + 1);
+            if (i0 > 0 && (i0 & BOR_CHUNK) == 0 && i < iend) {
+#pragma unroll
+                for (int m = 0; m < MB; ++m)
+                    z[m] = bor_unit((int)((unsigned)((n0 + 2 * m) * i) % (unsigned)N), N);
+            }
+            for (; i < iend; i += groups) {
+                const int j = i - i0;
+                const double2 v0 = set[j];
+                double2 v1, v2, v3, v4;
+                if constexpr (MFIE) {
+                    v1 = set[BOR_CHUNK + j];
+                    v2 = set[2 * BOR_CHUNK + j];
+                    v3 = set[3 * BOR_CHUNK + j];
+                    v4 = set[4 * BOR_CHUNK + j];
+                }
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    const double2 c = z[m];
+                    acc[m][0].x = fma(v0.x, c.x, acc[m][0].x);
+                    acc[m][0].y = fma(v0.y, c.x, acc[m][0].y);
+                    if constexpr (MFIE) {
+                        acc[m][1].x = fma(v1.x, c.x, acc[m][1].x);
+                        acc[m][1].y = fma(v1.y, c.x, acc[m][1].y);
+                        acc[m][2].x = fma(v2.x, c.y, acc[m][2].x);
+                        acc[m][2].y = fma(v2.y, c.y, acc[m][2].y);
+                        acc[m][3].x = fma(v3.x, c.y, acc[m][3].x);
+                        acc[m][3].y = fma(v3.y, c.y, acc[m][3].y);
+                        acc[m][4].x = fma(v4.x, c.x, acc[m][4].x);
+                        acc[m][4].y = fma(v4.y, c.x, acc[m][4].y);
                     }
+                    z[m] = make_double2(c.x * rot[m].x - c.y * rot[m].y, c.x * rot[m].y + c.y * rot[m].x);
                 }
             }
         }
-        if (grp < S) {
-            double2 *r = red + (grp * nm + n) * NV;
-            r[0] = sg;
-            if constexpr (MFIE) {
-                r[1] = s1;
-                r[2] = s2;
-                r[3] = s3;
-                r[4] = s4;
+#pragma unroll
+        for (int m = 0; m < MB; ++m) {
+            bor_sum_groups<NV>(acc[m], block, blocks, groups);
+            const int n = n0 + 2 * m;
+            if (grp == 0 && n < nm) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) sums[(pp * nm + n) * NV + v] = acc[m][v];
             }
-        }
-        __syncthreads();
-        for (int i = t; i < nm * NV; i += blockDim.x) {
-            double2 v = make_double2(0.0, 0.0);
-            for (int gq = 0; gq < S; ++gq) {
-                const double2 r = red[gq * nm * NV + i];
-                v.x += r.x;
-                v.y += r.y;
-            }
-            sums[pp * nm * NV + i] = v;
         }
     }
     __syncthreads();
@@ -290,9 +328,10 @@ k_bor_far(int ne, const double *__restrict__ nodes, const unsigned char *__restr
         const int nn_ = i / nsl, slot = i - nn_ * nsl;
         const int v = slot < BOR_SLOTS ? 0 : 1 + ((slot - BOR_SLOTS) >> 2);
         double2 a = make_double2(0.0, 0.0);
-        for (int pp = 0; pp < NPP; ++pp) {
-            const double fc = fac[pp * nsl + slot];
-            const double2 sv = sums[(pp * nm + nn_) * NV + v];
+#pragma unroll
+        for (int q = 0; q < BOR_FAR_PAIRS; ++q) {
+            const double fc = fac[q * nsl + slot];
+            const double2 sv = sums[(q * nm + nn_) * NV + v];
             a.x += fc * sv.x;
             a.y += fc * sv.y;
         }
@@ -307,11 +346,13 @@ k_bor_far(int ne, const double *__restrict__ nodes, const unsigned char *__restr
 }
 
 // Near-pair xi rule on [0, pi] for delta = R0 / c, span = 4 pi / (nmax + k c + 1) (two
-// periods of the fastest oscillation per panel):
-// a sinh-mapped Gauss core on [0, a], a = min(4 delta, span, pi), then panels
-// [a 2^g, a 2^(g+1)] while a 2^g < span, then panels of length span up to pi.
+// periods of the fastest oscillation): a sinh-mapped 20-point Gauss core on [0, a],
+// a = min(4 delta, span, pi); 16-point panels [a 2^g, a 2^(g+1)] while a 2^g < span; then
+// equal 32-point panels of at most four spans (eight periods, four points a period: the Gauss
+// error of such an oscillation, (pi P/2)^65 / 65! at P = 8, is below 1e-19, and the nearest
+// singularity, one span to the left, costs 2.6^-64) up to pi.
 struct BorRule {
-    double delta, span, a, vmax, top;
+    double delta, span, a, vmax, top, wide;
     int geo, uni;
 };
 
@@ -328,35 +369,54 @@ __device__ __forceinline__ BorRule bor_rule(double delta, double span) {
         ++r.geo;
     }
     r.top = top;
-    int uni = top < GRIM_PI ? (int)ceil((GRIM_PI - top) / span) : 0;
-    if (uni > 0 && top + (uni - 1) * span >= GRIM_PI) --uni;
-    r.uni = uni;
+    r.uni = top < GRIM_PI ? (int)ceil((GRIM_PI - top) / (4.0 * span)) : 0;
+    r.wide = r.uni > 0 ? (GRIM_PI - top) / r.uni : 0.0;
     return r;
 }
 
-__device__ __forceinline__ int bor_rule_count(const BorRule &r) { return BOR_XI_CORE + BOR_XI_PANEL * (r.geo + r.uni); }
+__device__ __forceinline__ int bor_rule_count(const BorRule &r) {
+    return BOR_XI_CORE + BOR_XI_PANEL * r.geo + BOR_XI_WIDE * r.uni;
+}
+
+// Gauss nodes and weights on [0, 1] of the rule's three orders, in shared memory (a constant
+// table is read one address at a time).
+struct BorGauss {
+    double x[BOR_XI_CORE + BOR_XI_PANEL + BOR_XI_WIDE], w[BOR_XI_CORE + BOR_XI_PANEL + BOR_XI_WIDE];
+};
+
+__device__ __forceinline__ void bor_gauss_fill(BorGauss &g) {
+    for (int i = threadIdx.x; i < BOR_XI_CORE + BOR_XI_PANEL + BOR_XI_WIDE; i += blockDim.x) {
+        const int q = i < BOR_XI_CORE ? BOR_XI_CORE : (i < BOR_XI_CORE + BOR_XI_PANEL ? BOR_XI_PANEL : BOR_XI_WIDE);
+        const int at = i - (q == BOR_XI_CORE ? 0 : (q == BOR_XI_PANEL ? BOR_XI_CORE : BOR_XI_CORE + BOR_XI_PANEL));
+        double x, w;
+        gl_node(q, at, x, w);
+        g.x[i] = 0.5 * (x + 1.0);
+        g.w[i] = 0.5 * w;
+    }
+}
 
 // Node j of the rule: xi and weight (times 2 for the half range).
-__device__ __forceinline__ void bor_rule_node(const BorRule &r, int j, double &xi, double &w) {
-    double x, wg;
+__device__ __forceinline__ void bor_rule_node(const BorRule &r, const BorGauss &g, int j, double &xi, double &w) {
     if (j < BOR_XI_CORE) {
-        gl_node(BOR_XI_CORE, j, x, wg);
-        const double v = 0.5 * (x + 1.0) * r.vmax;
+        const double v = g.x[j] * r.vmax;
         xi = r.delta * sinh(v);
-        w = r.delta * cosh(v) * (0.5 * wg) * r.vmax;
+        w = r.delta * cosh(v) * g.w[j] * r.vmax;
     } else {
-        const int P = (j - BOR_XI_CORE) / BOR_XI_PANEL, q = (j - BOR_XI_CORE) % BOR_XI_PANEL;
-        double lo, hi;
+        double lo, len;
+        int at;
+        const int jp = j - BOR_XI_CORE, P = jp / BOR_XI_PANEL;
         if (P < r.geo) {
+            at = BOR_XI_CORE + jp % BOR_XI_PANEL;
             lo = ldexp(r.a, P);
-            hi = fmin(ldexp(r.a, P + 1), GRIM_PI);
+            len = fmin(ldexp(r.a, P + 1), GRIM_PI) - lo;
         } else {
-            lo = fmin(r.top + (P - r.geo) * r.span, GRIM_PI);
-            hi = fmin(r.top + (P + 1 - r.geo) * r.span, GRIM_PI);
+            const int ju = jp - BOR_XI_PANEL * r.geo;
+            at = BOR_XI_CORE + BOR_XI_PANEL + ju % BOR_XI_WIDE;
+            lo = fma((double)(ju / BOR_XI_WIDE), r.wide, r.top);
+            len = r.wide;
         }
-        gl_node(BOR_XI_PANEL, q, x, wg);
-        xi = lo + (hi - lo) * (0.5 * (x + 1.0));
-        w = (hi - lo) * (0.5 * wg);
+        xi = fma(len, g.x[at], lo);
+        w = len * g.w[at];
     }
     w *= 2.0;
 }
@@ -365,123 +425,138 @@ struct BorItem {
     int e, f, r0, r1;  // element pair and its point-pair range in the rule table
 };
 
-#define BOR_NEAR_EVAL 256  // near-rule samples evaluated per pass (one per thread)
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// Stride of a sample's row of starting phases (not a multiple of 8: sixteen-byte words of
+// eight rows in eight banks groups).
+__host__ __device__ constexpr int bor_near_stride(int blocks) { return blocks % 8 == 0 ? blocks + 1 : blocks; }
+// Complex words of a warp's staging area; its point pair's sums [nm][NV] reuse it.
+__host__ __device__ constexpr int bor_near_area(int nm, int nv, int blocks) {
+    return BOR_CHUNK * (nv + 1 + bor_near_stride(blocks)) > nm * nv ? BOR_CHUNK * (nv + 1 + bor_near_stride(blocks))
+                                                                    : nm * nv;
 }
 
-// grid = number of near work items, BOR_THREADS threads.  rule[3 i .. 3 i + 2] = (s, s', w).
-// Writes the item's moments to part[item][n][slot] (nm x nsl complex).  Per point pair the
-// rule's samples are evaluated BOR_NEAR_EVAL at a time (one per thread, with e^{j xi} and
-// e^{j Q xi}, Q = ceil(nm / 4)); rows e^{j n xi} of chr samples at a time are then built by
-// rotation (four threads per sample, one quarter of the orders each) and summed by the
-// (mode, group) threads.
-// dynamic smem: smp[NV][BOR_NEAR_EVAL], z1[BOR_NEAR_EVAL], zq[BOR_NEAR_EVAL],
-// rot[chr][P] (P = nm rounded up to odd: conflict-free row writes; the groups' partial
-// sums red[S][nm][NV] reuse it once a point pair's rows are consumed), then sum, acc, fac.
-template <bool MFIE>
-__global__ void __launch_bounds__(BOR_THREADS, 2)
+// grid = number of near work items, at most BOR_NEAR_WARPS warps.  rule[3 i .. 3 i + 2] = (s, s', w).
+// Writes the item's moments to part[item][n][slot] (nm x nsl complex).  Each warp takes its
+// share of the point pairs: BOR_CHUNK samples at a time, one per lane with e^{j xi} and the phases
+// e^{j n xi} at the start n of every block, then each lane the orders of its block.  After
+// every round of one point pair a warp the CTA folds their sums into the item's moments.
+// dynamic smem: area[warp], acc[nm][nsl], fac[warp][nsl], Gauss nodes.
+template <bool MFIE, int MB>
+__global__ void __launch_bounds__(32 * BOR_NEAR_WARPS, 2)
 k_bor_near(const BorItem *__restrict__ items, const double *__restrict__ nodes, const double *__restrict__ rule,
-           double k, int mmax, int chr, double2 *__restrict__ part) {
+           double k, int mmax, double2 *__restrict__ part) {
     constexpr int NV = MFIE ? 5 : 1, nsl = MFIE ? BOR_ALL_SLOTS : BOR_SLOTS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int nm = mmax + 2, S = BOR_THREADS / nm, P = nm | 1, Q = (nm + 3) / 4;
-    double2 *smp = reinterpret_cast<double2 *>(smem_raw);  // [NV][BOR_NEAR_EVAL]
-    double2 *sz1 = smp + NV * BOR_NEAR_EVAL;
-    double2 *szq = sz1 + BOR_NEAR_EVAL;
-    double2 *rot = szq + BOR_NEAR_EVAL;                     // [chr][P]
-    double2 *red = rot;                                     // [S][nm][NV], after the rows
-    double2 *sum = rot + max(chr * P, S * nm * NV);
-    double2 *acc = sum + nm * NV;
+    const int nm = mmax + 2, t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = blockDim.x >> 5;
+    const int blocks = bor_near_blocks(nm, MB), groups = 32 / blocks, P = bor_near_stride(blocks);
+    const int area = bor_near_area(nm, NV, blocks);
+    double2 *areas = reinterpret_cast<double2 *>(smem_raw);
+    double2 *smp = areas + warp * area;           // [NV][BOR_CHUNK]
+    double2 *z1 = smp + NV * BOR_CHUNK;           // [BOR_CHUNK]
+    double2 *zt = z1 + BOR_CHUNK;                 // [BOR_CHUNK][P]
+    double2 *acc = areas + warps * area;           // [nm][nsl]
     double *fac = reinterpret_cast<double *>(acc + nm * nsl);
+    BorGauss &gauss = *reinterpret_cast<BorGauss *>(fac + warps * nsl);
     const BorItem it = items[blockIdx.x];
-    const int t = threadIdx.x, n = t % nm, grp = t / nm;
+    const int block = lane % blocks, grp = lane / blocks, n0 = block * MB;
+    bor_gauss_fill(gauss);
     for (int i = t; i < nm * nsl; i += blockDim.x) acc[i] = make_double2(0.0, 0.0);
-    for (int ipp = it.r0; ipp < it.r1; ++ipp) {
-        const BorPt p = bor_point(nodes, it.e, rule[3 * ipp], rule[3 * ipp + 2]);
-        const BorPt q = bor_point(nodes, it.f, rule[3 * ipp + 1], 1.0);
-        const BorPair pr = bor_pair(k, p, q);
-        const double c = sqrt(p.rho * q.rho);
-        const BorRule rl = bor_rule(sqrt(pr.d2) / c, 4.0 * GRIM_PI / ((mmax + 1) + k * c + 1.0));
-        const int na = bor_rule_count(rl);
-        if (t < nsl) fac[t] = bor_factor(p, q, t);
-        double2 sg = make_double2(0.0, 0.0), s1 = sg, s2 = sg, s3 = sg, s4 = sg;
-        for (int j0 = 0; j0 < na; j0 += BOR_NEAR_EVAL) {
-            const int cnt = min(BOR_NEAR_EVAL, na - j0);
-            __syncthreads();
-            for (int j = t; j < cnt; j += blockDim.x) {
-                double xi, w;
-                bor_rule_node(rl, j0 + j, xi, w);
-                double sh, ch;
-                sincos(0.5 * xi, &sh, &ch);
-                double2 g, F[4];
-                bor_sample<MFIE>(pr, sh, 2.0 * sh * ch, w, g, F);
-                smp[j] = g;
-                if constexpr (MFIE) {
+    __syncthreads();
+    for (int base = it.r0; base < it.r1; base += warps) {
+        const int ipp = base + warp;
+        if (ipp < it.r1) {
+            const BorPt p = bor_point(nodes, it.e, rule[3 * ipp], rule[3 * ipp + 2]);
+            const BorPt q = bor_point(nodes, it.f, rule[3 * ipp + 1], 1.0);
+            const BorPair pr = bor_pair(k, p, q);
+            const double c = sqrt(p.rho * q.rho);
+            const BorRule rl = bor_rule(sqrt(pr.d2) / c, 4.0 * GRIM_PI / ((mmax + 1) + k * c + 1.0));
+            const int na = bor_rule_count(rl);
+            for (int s = lane; s < nsl; s += 32) fac[warp * nsl + s] = bor_factor(p, q, s);
+            double2 sum[MB][NV];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) smp[(1 + u) * BOR_NEAR_EVAL + j] = F[u];
-                }
-                // e^{j xi} and e^{j Q xi} (binary powers)
-                const double2 z1 = make_double2(1.0 - 2.0 * sh * sh, 2.0 * sh * ch);
-                double2 zq = make_double2(1.0, 0.0), b = z1;
-                for (int e2 = Q; e2 > 0; e2 >>= 1) {
-                    if (e2 & 1) zq = cmul(zq, b);
-                    b = cmul(b, b);
-                }
-                sz1[j] = z1;
-                szq[j] = zq;
-            }
-            for (int s0 = 0; s0 < cnt; s0 += chr) {
-                const int sc = min(chr, cnt - s0);
-                __syncthreads();
-                for (int task = t; task < 4 * sc; task += blockDim.x) {
-                    const int jj = task % sc, quarter = task / sc;
-                    const int n0 = quarter * Q, n1 = min(nm, n0 + Q);
-                    if (n0 >= n1) continue;
-                    const double2 z1 = sz1[s0 + jj], zq = szq[s0 + jj];
-                    double2 z = make_double2(1.0, 0.0);
-                    for (int r = 0; r < quarter; ++r) z = cmul(z, zq);
-                    double2 *row = rot + jj * P;
-                    for (int nn_ = n0; nn_ < n1; ++nn_) {
-                        row[nn_] = z;
-                        z = cmul(z, z1);
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int v = 0; v < NV; ++v) sum[m][v] = make_double2(0.0, 0.0);
+            for (int j0 = 0; j0 < na; j0 += BOR_CHUNK) {
+                const int cnt = min(BOR_CHUNK, na - j0);
+                __syncwarp();
+                if (lane < cnt) {
+                    double xi, w, sh, ch;
+                    bor_rule_node(rl, gauss, j0 + lane, xi, w);
+                    gh_sincos(0.5 * xi, sh, ch);
+                    double2 g, F[4];
+                    bor_sample<MFIE>(pr, sh, 2.0 * sh * ch, w, g, F);
+                    smp[lane] = g;
+                    if constexpr (MFIE) {
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) smp[(1 + v) * BOR_CHUNK + lane] = F[v];
+                    }
+                    const double2 u = make_double2(1.0 - 2.0 * sh * sh, 2.0 * sh * ch);
+                    z1[lane] = u;
+                    double2 step = cmul(u, u), z = make_double2(1.0, 0.0);
+                    step = MB == 4 ? cmul(step, step) : cmul(step, u);
+                    for (int b = 0; b < blocks; ++b) {
+                        zt[lane * P + b] = z;
+                        z = cmul(z, step);
                     }
                 }
-                __syncthreads();
-                if (grp < S) {
-#pragma unroll 4
-                    for (int jj = grp; jj < sc; jj += S) {
-                        const double2 z = rot[jj * P + n];
-                        const int j = s0 + jj;
-                        const double2 v = smp[j];
-                        sg.x += v.x * z.x;
-                        sg.y += v.y * z.x;
+                __syncwarp();
+                if (grp < groups) {
+                    for (int j = grp; j < cnt; j += groups) {
+                        const double2 u = z1[j], v0 = smp[j];
+                        double2 z = zt[j * P + block], v1, v2, v3, v4;
                         if constexpr (MFIE) {
-                            const double2 f0 = smp[BOR_NEAR_EVAL + j], f1 = smp[2 * BOR_NEAR_EVAL + j];
-                            const double2 f2 = smp[3 * BOR_NEAR_EVAL + j], f3 = smp[4 * BOR_NEAR_EVAL + j];
-                            s1.x += f0.x * z.x; s1.y += f0.y * z.x;
-                            s2.x += f1.x * z.y; s2.y += f1.y * z.y;
-                            s3.x += f2.x * z.y; s3.y += f2.y * z.y;
-                            s4.x += f3.x * z.x; s4.y += f3.y * z.x;
+                            v1 = smp[BOR_CHUNK + j];
+                            v2 = smp[2 * BOR_CHUNK + j];
+                            v3 = smp[3 * BOR_CHUNK + j];
+                            v4 = smp[4 * BOR_CHUNK + j];
+                        }
+#pragma unroll
+                        for (int m = 0; m < MB; ++m) {
+                            sum[m][0].x = fma(v0.x, z.x, sum[m][0].x);
+                            sum[m][0].y = fma(v0.y, z.x, sum[m][0].y);
+                            if constexpr (MFIE) {
+                                sum[m][1].x = fma(v1.x, z.x, sum[m][1].x);
+                                sum[m][1].y = fma(v1.y, z.x, sum[m][1].y);
+                                sum[m][2].x = fma(v2.x, z.y, sum[m][2].x);
+                                sum[m][2].y = fma(v2.y, z.y, sum[m][2].y);
+                                sum[m][3].x = fma(v3.x, z.y, sum[m][3].x);
+                                sum[m][3].y = fma(v3.y, z.y, sum[m][3].y);
+                                sum[m][4].x = fma(v4.x, z.x, sum[m][4].x);
+                                sum[m][4].y = fma(v4.y, z.x, sum[m][4].y);
+                            }
+                            if (m + 1 < MB) z = cmul(z, u);
                         }
                     }
                 }
             }
-        }
-        __syncthreads();  // every thread is done with the rows that red overwrites
-        if (grp < S) {
-            double2 *r = red + (grp * nm + n) * NV;
-            r[0] = sg;
-            if constexpr (MFIE) {
-                r[1] = s1;
-                r[2] = s2;
-                r[3] = s3;
-                r[4] = s4;
+            __syncwarp();  // the samples are consumed: the sums take their place
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+                bor_sum_groups<NV>(sum[m], block, blocks, groups);
+                if (grp == 0 && n0 + m < nm) {
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) smp[(n0 + m) * NV + v] = sum[m][v];
+                }
             }
         }
         __syncthreads();
-        bor_fold_pair<MFIE>(nm, S, red, sum, fac, acc);
+        const int cnt = min(warps, it.r1 - base);
+        for (int i = t; i < nm * nsl; i += blockDim.x) {
+            const int n = i / nsl, slot = i - n * nsl, v = slot < BOR_SLOTS ? 0 : 1 + ((slot - BOR_SLOTS) >> 2);
+            double2 a = make_double2(0.0, 0.0);
+            for (int w = 0; w < cnt; ++w) {
+                const double f = fac[w * nsl + slot];
+                const double2 s = areas[w * area + n * NV + v];
+                a.x = fma(f, s.x, a.x);
+                a.y = fma(f, s.y, a.y);
+            }
+            // odd brackets: K = -j sum F sin(n xi)
+            if (v == 2 || v == 3) a = make_double2(a.y, -a.x);
+            acc[i].x += a.x;
+            acc[i].y += a.y;
+        }
+        __syncthreads();
     }
     double2 *out = part + (int64_t)blockIdx.x * nm * nsl;
     for (int i = t; i < nm * nsl; i += blockDim.x) out[i] = acc[i];

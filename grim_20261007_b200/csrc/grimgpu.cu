@@ -2782,24 +2782,19 @@ extern "C" int64_t grim_bor_mfie_moments_size(int ne, int mmax) {
     return (int64_t)ne * ne * (mmax + 2) * BOR_KSLOTS * (int64_t)sizeof(double2);
 }
 
-template <bool MFIE>
-static size_t bor_tail_smem(int nm) {
-    const int NV = MFIE ? 5 : 1, nsl = MFIE ? BOR_ALL_SLOTS : BOR_SLOTS, S = BOR_THREADS / nm;
-    return sizeof(double2) * ((size_t)S * nm * NV + (size_t)nm * NV + (size_t)nm * nsl) + sizeof(double) * nsl;
-}
-
-template <bool MFIE>
+template <bool MFIE, int MB>
 static int bor_moments_launch(grim_context *h, int ne, const double *nodes, const unsigned char *d_cls, double k,
                               int mmax, int nxi_cap, const std::vector<BorItem> &items,
                               const std::vector<int4> &pairs, const double *d_rule, double2 *mom, double2 *momk) {
     const int nm = mmax + 2, NV = MFIE ? 5 : 1, nsl = MFIE ? BOR_ALL_SLOTS : BOR_SLOTS;
     // far pairs
-    const int S = BOR_THREADS / nm, NPP = BOR_FAR_ORDER * BOR_FAR_ORDER;
-    const size_t far_smem = sizeof(double2) * ((size_t)NV * BOR_FAR_CHUNK + (size_t)S * nm * NV + (size_t)NPP * nm * NV) +
-                            sizeof(double) * NPP * nsl;
-    GRIM_CHECK_CUDA(cudaFuncSetAttribute(k_bor_far<MFIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)far_smem));
-    k_bor_far<MFIE><<<dim3(ne, ne), BOR_THREADS, far_smem, h->stream>>>(ne, nodes, d_cls, k, mmax, nxi_cap, mom,
-                                                                          momk);
+    const size_t far_smem =
+        sizeof(double2) * ((size_t)BOR_FAR_WARPS * 2 * NV * BOR_CHUNK + (size_t)BOR_FAR_PAIRS * nm * NV) +
+        sizeof(double) * BOR_FAR_PAIRS * nsl;
+    GRIM_CHECK_CUDA(
+        cudaFuncSetAttribute(k_bor_far<MFIE, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)far_smem));
+    k_bor_far<MFIE, MB><<<dim3(ne, ne), 32 * BOR_FAR_WARPS, far_smem, h->stream>>>(ne, nodes, d_cls, k, mmax, nxi_cap,
+                                                                                   mom, momk);
     GRIM_CHECK_LAUNCH(h, MFIE ? "k_bor_far<cfie>" : "k_bor_far<efie>");
     if (items.empty()) return GRIM_OK;
     void *p_items = nullptr, *p_pairs = nullptr, *p_part = nullptr;
@@ -2810,14 +2805,18 @@ static int bor_moments_launch(grim_context *h, int ne, const double *nodes, cons
                                     h->stream));
     GRIM_CHECK_CUDA(cudaMemcpyAsync(p_pairs, pairs.data(), pairs.size() * sizeof(int4), cudaMemcpyHostToDevice,
                                     h->stream));
-    const int chr = nm <= 64 ? 64 : 32;
-    // rows and the groups' partial sums share one region (red = S nm NV complex)
-    const size_t near_smem = sizeof(double2) * ((size_t)(NV + 2) * BOR_NEAR_EVAL +
-                                                std::max((size_t)chr * (nm | 1), (size_t)S * nm * NV)) +
-                             bor_tail_smem<MFIE>(nm) - sizeof(double2) * (size_t)S * nm * NV;
-    GRIM_CHECK_CUDA(cudaFuncSetAttribute(k_bor_near<MFIE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)near_smem));
-    k_bor_near<MFIE><<<(unsigned)items.size(), BOR_THREADS, near_smem, h->stream>>>(
-        (const BorItem *)p_items, nodes, d_rule, k, mmax, chr, (double2 *)p_part);
+    // eight warps, or as many as leave room for the item's moments (128 orders: six)
+    auto near_bytes = [&](int warps) {
+        return sizeof(double2) * ((size_t)warps * bor_near_area(nm, NV, bor_near_blocks(nm, MB)) + (size_t)nm * nsl) +
+               sizeof(double) * warps * nsl + sizeof(BorGauss);
+    };
+    int warps = BOR_NEAR_WARPS;
+    while (warps > 1 && near_bytes(warps) > (size_t)226 * 1024) --warps;
+    const size_t near_smem = near_bytes(warps);
+    GRIM_CHECK_CUDA(
+        cudaFuncSetAttribute(k_bor_near<MFIE, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)near_smem));
+    k_bor_near<MFIE, MB><<<(unsigned)items.size(), 32 * warps, near_smem, h->stream>>>(
+        (const BorItem *)p_items, nodes, d_rule, k, mmax, (double2 *)p_part);
     GRIM_CHECK_LAUNCH(h, MFIE ? "k_bor_near<cfie>" : "k_bor_near<efie>");
     k_bor_near_reduce<MFIE><<<(unsigned)pairs.size(), 256, 0, h->stream>>>(ne, mmax, (const int4 *)p_pairs,
                                                                            (const double2 *)p_part, mom, momk);
@@ -2862,13 +2861,11 @@ extern "C" int grim_bor_moments(grim_handle_t h, int ne, const double *nodes, do
     if (h->profiling) grim_prof_mark(h, "bor_upload", 0, 0);
     // a multiple of 32 keeps the shared-memory sections after the sample table 16-byte aligned
     const int cap = std::min(BOR_MAX_NXI, (std::max(32, nxi_max) + 31) / 32 * 32);
-    int s;
-    if (mom_k)
-        s = bor_moments_launch<true>(h, ne, nodes, (const unsigned char *)p_cls, k, mmax, cap, items, pairs,
-                                     (const double *)p_rule, (double2 *)mom, (double2 *)mom_k);
-    else
-        s = bor_moments_launch<false>(h, ne, nodes, (const unsigned char *)p_cls, k, mmax, cap, items, pairs,
-                                      (const double *)p_rule, (double2 *)mom, nullptr);
+    const bool three = bor_mb(mmax + 2) == 3;
+    auto launch = mom_k ? (three ? bor_moments_launch<true, 3> : bor_moments_launch<true, 4>)
+                        : (three ? bor_moments_launch<false, 3> : bor_moments_launch<false, 4>);
+    const int s = launch(h, ne, nodes, (const unsigned char *)p_cls, k, mmax, cap, items, pairs, (const double *)p_rule,
+                         (double2 *)mom, (double2 *)mom_k);
     GRIM_TRY(s);
     // the host vectors above are freed on return: wait for the uploads that read them
     GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));

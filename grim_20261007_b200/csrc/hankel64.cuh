@@ -250,6 +250,15 @@ __host__ __device__ __forceinline__ void gh_combine(const double (&v)[4], double
     h = make_double2(fma(Bs, q1, -Bc * v[2]), fma(Bs, v[2], Bc * q1));
 }
 
+// Sine and cosine of x, |x| < 2^30: x = n pi/2 + r in two parts, then the polynomials.
+__host__ __device__ __forceinline__ void gh_sincos(double x, double &sn, double &cs) {
+    const double shift = 6755399441055744.0;
+    const double t = fma(x, 0.63661977236758134308, shift), m = t - shift;
+    double r = fma(-m, 1.57079632679489661923, x);
+    r = fma(-m, 6.1232339957367658862e-17, r);
+    gh_sincos_quadrant(r, gh_low_word(t), sn, cs);
+}
+
 __host__ __device__ __noinline__ static void hankel_pair_library(double u, double2 &g, double2 &h) {
     const double x = sqrt(u);
     g = make_double2(0.25 * y0(x), 0.25 * j0(x));
