@@ -159,6 +159,10 @@ struct grim_context {
     cudaGraphExec_t grp_exec = nullptr;
     std::vector<int64_t> grp_key;
     int64_t grp_graph_launches = 0;
+    // host copies (hoststage.cuh): pinned slots, an event per slot and whether it is pending
+    void *stage = nullptr;
+    std::vector<cudaEvent_t> stage_events;
+    std::vector<char> stage_pending;
     // profiling: one event per launch (plus a start event), aggregated by kernel name
     int profiling = 0;
     cudaEvent_t prof_start = nullptr;

@@ -29,6 +29,7 @@
 #include "gepp_loop.cuh"
 #include "condest.cuh"
 #include "modecond.cuh"
+#include "hoststage.cuh"
 
 // ============================================================== errors
 static thread_local std::string g_last_error;
@@ -182,6 +183,7 @@ extern "C" int grim_release_workspace(grim_handle_t h) {
     DeviceGuard g(h->device);
     for (auto &kv : h->ws) cudaFreeAsync(kv.second.first, h->stream);
     h->ws.clear();
+    stage_free(h);
     GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));
     if (h->grp_exec) {  // the captured grouped factorization read the freed buffers
         cudaGraphExecDestroy(h->grp_exec);
@@ -2628,7 +2630,7 @@ extern "C" int grim_far_block(grim_handle_t h, int64_t mb, int64_t nb, int q, in
 // ghost_far_block (twod/assembly/native/far.c:193-207, loaded by
 // twod/assembly/native/far.py:184-199): copies in, runs grim_far_block on the calling
 // thread's own handle (current device), copies the accumulators back.  Thread-safe.
-extern "C" int ghost_far_block(int64_t mb, int64_t nb, int q, int width, const double *obs_pts,
+static int far_block_host(bool fresh, int64_t mb, int64_t nb, int q, int width, const double *obs_pts,
                                const double *src_pts, const double *qw, const double *phi, const double *obs_norm,
                                const double *src_norm, const uint8_t *far, int obs_normal_deriv, int want_s,
                                int want_k, int mirrored, double k_re, double k_im, int intervals,
@@ -2660,33 +2662,51 @@ extern "C" int ghost_far_block(int64_t mb, int64_t nb, int q, int width, const d
     double *d_as = (double *)(((uintptr_t)(d_c + tab_c) + 255) & ~(uintptr_t)255);
     double *d_ak = (double *)((char *)d_as + acc_bytes), *d_akt = (double *)((char *)d_ak + acc_bytes);
     uint8_t *d_far = (uint8_t *)((char *)d_akt + acc_bytes);
-    auto up = [&](void *dst, const void *src, size_t n) {
-        return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, h->stream);
-    };
-    GRIM_CHECK_CUDA(up(d_op, obs_pts, pts_o * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_sp, src_pts, pts_s * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_qw, qw, q * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_phi, phi, (size_t)q * width * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_on, obs_norm, 2 * mb * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_sn, src_norm, 2 * nb * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_b, bounds, (intervals + 1) * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_c, coeff, tab_c * sizeof(double)));
-    GRIM_CHECK_CUDA(up(d_far, far, (size_t)mb * nb));
-    if (want_s) GRIM_CHECK_CUDA(up(d_as, acc_s, acc_bytes));
-    if (want_k) GRIM_CHECK_CUDA(up(d_ak, acc_k, acc_bytes));
-    if (with_kt) GRIM_CHECK_CUDA(up(d_akt, acc_kt, acc_bytes));
+    std::vector<HostCopy> in;
+    auto up = [&](void *dst, const void *src, size_t n) { in.push_back({dst, const_cast<void *>(src), n}); };
+    up(d_op, obs_pts, pts_o * sizeof(double));
+    up(d_sp, src_pts, pts_s * sizeof(double));
+    up(d_qw, qw, q * sizeof(double));
+    up(d_phi, phi, (size_t)q * width * sizeof(double));
+    up(d_on, obs_norm, 2 * mb * sizeof(double));
+    up(d_sn, src_norm, 2 * nb * sizeof(double));
+    up(d_b, bounds, (intervals + 1) * sizeof(double));
+    up(d_c, coeff, tab_c * sizeof(double));
+    up(d_far, far, (size_t)mb * nb);
+    std::vector<HostCopy> acc;
+    if (want_s) acc.push_back({d_as, acc_s, acc_bytes});
+    if (want_k) acc.push_back({d_ak, acc_k, acc_bytes});
+    if (with_kt) acc.push_back({d_akt, acc_kt, acc_bytes});
+    if (!fresh) in.insert(in.end(), acc.begin(), acc.end());
+    GRIM_TRY(stage_copy(h, in, true));
+    if (fresh)
+        for (const HostCopy &c : acc) GRIM_CHECK_CUDA(cudaMemsetAsync(c.device, 0, c.bytes, h->stream));
     const int s = grim_far_block(h, mb, nb, q, width, d_op, d_sp, d_qw, d_phi, d_on, d_sn, d_far, obs_normal_deriv,
                                  want_s, want_k, mirrored, k_re, k_im, intervals, d_b, degree, d_c,
                                  want_s ? d_as : nullptr, want_k ? d_ak : nullptr, with_kt ? d_akt : nullptr);
     if (s != GRIM_OK) return s;
-    auto down = [&](void *dst, const void *src, size_t n) {
-        return cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, h->stream);
-    };
-    if (want_s) GRIM_CHECK_CUDA(down(acc_s, d_as, acc_bytes));
-    if (want_k) GRIM_CHECK_CUDA(down(acc_k, d_ak, acc_bytes));
-    if (with_kt) GRIM_CHECK_CUDA(down(acc_kt, d_akt, acc_bytes));
-    GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));
-    return 0;
+    return stage_copy(h, acc, false);
+}
+
+extern "C" int ghost_far_block(int64_t mb, int64_t nb, int q, int width, const double *obs_pts,
+                               const double *src_pts, const double *qw, const double *phi, const double *obs_norm,
+                               const double *src_norm, const uint8_t *far, int obs_normal_deriv, int want_s,
+                               int want_k, int mirrored, double k_re, double k_im, int intervals,
+                               const double *bounds, int degree, const double *coeff, double *acc_s, double *acc_k,
+                               double *acc_kt) {
+    return far_block_host(false, mb, nb, q, width, obs_pts, src_pts, qw, phi, obs_norm, src_norm, far, obs_normal_deriv, want_s, want_k,
+                          mirrored, k_re, k_im, intervals, bounds, degree, coeff, acc_s, acc_k, acc_kt);
+}
+
+// ghost_far_block into accumulators that hold nothing yet: they are not copied in.
+extern "C" int grim_far_block_fresh(int64_t mb, int64_t nb, int q, int width, const double *obs_pts,
+                               const double *src_pts, const double *qw, const double *phi, const double *obs_norm,
+                               const double *src_norm, const uint8_t *far, int obs_normal_deriv, int want_s,
+                               int want_k, int mirrored, double k_re, double k_im, int intervals,
+                               const double *bounds, int degree, const double *coeff, double *acc_s, double *acc_k,
+                               double *acc_kt) {
+    return far_block_host(true, mb, nb, q, width, obs_pts, src_pts, qw, phi, obs_norm, src_norm, far, obs_normal_deriv, want_s, want_k,
+                          mirrored, k_re, k_im, intervals, bounds, degree, coeff, acc_s, acc_k, acc_kt);
 }
 
 // B1 drop-in with host buffers.
@@ -2698,16 +2718,49 @@ extern "C" int grim_zgesv_batched(grim_handle_t h, int n, int nrhs, const double
     void *pa = nullptr, *pb = nullptr;
     GRIM_TRY(grim_workspace(h, "h_A", (size_t)n * n * sizeof(double2), &pa));
     GRIM_TRY(grim_workspace(h, "h_B", (size_t)n * nrhs * sizeof(double2), &pb));
-    GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pa, n * sizeof(double2), A, (size_t)lda * sizeof(double2), n * sizeof(double2), n,
-                                      cudaMemcpyHostToDevice, h->stream));
-    GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pb, n * sizeof(double2), B, (size_t)ldb * sizeof(double2), n * sizeof(double2),
-                                      nrhs, cudaMemcpyHostToDevice, h->stream));
+    if (lda == n && ldb == n) {
+        GRIM_TRY(stage_copy(h, {{pa, const_cast<double *>(A), (size_t)n * n * sizeof(double2)},
+                                {pb, B, (size_t)n * nrhs * sizeof(double2)}}, true));
+    } else {
+        GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pa, n * sizeof(double2), A, (size_t)lda * sizeof(double2),
+                                          n * sizeof(double2), n, cudaMemcpyHostToDevice, h->stream));
+        GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pb, n * sizeof(double2), B, (size_t)ldb * sizeof(double2),
+                                          n * sizeof(double2), nrhs, cudaMemcpyHostToDevice, h->stream));
+    }
     int s = grim_zgesv_mixed(h, n, nrhs, pa, n, nullptr, 0, pb, n, precision_mode, 2e-12, 10, info, nullptr);
     if (s != GRIM_OK) return s;
+    if (ldb == n) return stage_copy(h, {{pb, B, (size_t)n * nrhs * sizeof(double2)}}, false);
     GRIM_CHECK_CUDA(cudaMemcpy2DAsync(B, (size_t)ldb * sizeof(double2), pb, n * sizeof(double2), n * sizeof(double2),
                                       nrhs, cudaMemcpyDeviceToHost, h->stream));
     GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));
     return GRIM_OK;
+}
+
+// The same for row-major (C-order) A (n x n), B and X (n x nrhs), B kept: the transposes that
+// a column-major call costs the host (3 ms at n = 900) run on the device.
+extern "C" int grim_zgesv_rowmajor(grim_handle_t h, int n, int nrhs, const double *A, const double *B, double *X,
+                                   int precision_mode, int *info) {
+    if (!h || n <= 0 || nrhs <= 0 || !A || !B || !X)
+        return grim_fail(GRIM_ERR_ARGUMENT, "grim_zgesv_rowmajor: bad arguments");
+    DeviceGuard g(h->device);
+    const size_t an = (size_t)n * n, bn = (size_t)n * nrhs;
+    void *pr = nullptr, *pa = nullptr, *pb = nullptr;
+    GRIM_TRY(grim_workspace(h, "h_rows", (an + bn) * sizeof(double2), &pr));
+    GRIM_TRY(grim_workspace(h, "h_A", an * sizeof(double2), &pa));
+    GRIM_TRY(grim_workspace(h, "h_B", bn * sizeof(double2), &pb));
+    double2 *ra = (double2 *)pr, *rb = ra + an;
+    GRIM_TRY(stage_copy(h, {{ra, const_cast<double *>(A), an * sizeof(double2)},
+                            {rb, const_cast<double *>(B), bn * sizeof(double2)}}, true));
+    const dim3 block(32, 8);
+    k_transpose<<<dim3(ceil_div(n, 32), ceil_div(n, 32)), block, 0, h->stream>>>(n, n, ra, n, (double2 *)pa, n);
+    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    k_transpose<<<dim3(ceil_div(nrhs, 32), ceil_div(n, 32)), block, 0, h->stream>>>(n, nrhs, rb, nrhs, (double2 *)pb, n);
+    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    GRIM_TRY(grim_zgesv_mixed(h, n, nrhs, pa, n, nullptr, 0, pb, n, precision_mode, 2e-12, 10, info, nullptr));
+    k_transpose<<<dim3(ceil_div(n, 32), ceil_div(nrhs, 32)), block, 0, h->stream>>>(nrhs, n, (const double2 *)pb, n, rb,
+                                                                                    nrhs);
+    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    return stage_copy(h, {{rb, X, bn * sizeof(double2)}}, false);
 }
 
 // ============================================================== profiling

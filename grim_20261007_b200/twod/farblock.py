@@ -4,10 +4,11 @@
 ``twod/assembly/native/far.py:201-249`` ``far_block``: accumulators (width^2, mb, nb)
 complex128 for S, K and the mirrored K of the far pairs (zero elsewhere), or None when a
 far distance falls below the kernel table (the caller then takes its NumPy path).  The
-work runs in ``ghost_far_block`` of libgrimgpu (``include/grimgpu.h``), which has the exact
-C signature of the reference's ``far.c:193`` export, so the reference can also load the
-library directly in place of its ``libghost_far.so``.  Results inside the table equal the
-reference's bit for bit (same operations in the same order, no fused multiply-add).
+work runs in libgrimgpu's ``grim_far_block_fresh``: its ``ghost_far_block`` with the sums
+starting from zero.  ``ghost_far_block`` (``include/grimgpu.h``) has the exact C signature of
+the reference's ``far.c:193`` export, so the reference can also load the library directly in
+place of its ``libghost_far.so``.  Results inside the table equal the reference's bit for bit
+(same operations in the same order, no fused multiply-add).
 """
 from __future__ import annotations
 
@@ -43,20 +44,21 @@ def far_block(table, k, obs_pts, src_pts, weights, phi, obs_normals, src_normals
     k = complex(k)
 
     def buffer(wanted):
-        return np.zeros((width * width, mb, nb), dtype=np.complex128) if wanted else None
+        return np.empty((width * width, mb, nb), dtype=np.complex128) if wanted else None
     acc_s, acc_k, acc_kt = buffer(want_s), buffer(want_k), buffer(want_k and mirrored)
     lib = _lib.load()
-    status = lib.ghost_far_block(mb, nb, q, width, obs_pts.ctypes.data, src_pts.ctypes.data, weights.ctypes.data,
-                                 phi.ctypes.data, obs_normals.ctypes.data, src_normals.ctypes.data, far.ctypes.data,
-                                 int(bool(obs_normal_deriv)), int(bool(want_s)), int(bool(want_k)),
-                                 int(bool(mirrored)), k.real, k.imag, len(bounds) - 1, bounds.ctypes.data,
-                                 coeff.shape[1] - 1, coeff.ctypes.data,
-                                 *(None if a is None else a.ctypes.data for a in (acc_s, acc_k, acc_kt)))
+    # the sums start from zero here: the accumulators only come down
+    status = lib.grim_far_block_fresh(mb, nb, q, width, obs_pts.ctypes.data, src_pts.ctypes.data,
+                                      weights.ctypes.data, phi.ctypes.data, obs_normals.ctypes.data,
+                                      src_normals.ctypes.data, far.ctypes.data, int(bool(obs_normal_deriv)),
+                                      int(bool(want_s)), int(bool(want_k)), int(bool(mirrored)), k.real, k.imag,
+                                      len(bounds) - 1, bounds.ctypes.data, coeff.shape[1] - 1, coeff.ctypes.data,
+                                      *(None if a is None else a.ctypes.data for a in (acc_s, acc_k, acc_kt)))
     if status == 2:
         return None
     if status == 3:
         raise RuntimeError('Far-block quadrature rejected its inputs.')
-    _lib.check(status, 'ghost_far_block')
+    _lib.check(status, 'grim_far_block_fresh')
     return acc_s, acc_k, acc_kt
 
 

@@ -130,21 +130,34 @@ def _solve_dense_gpu(a_eval, rhs_eval):
             f'GPU dense solve needs an estimated {required / 1024.0 ** 3:.3f} GiB, exceeding 80% of the '
             f'{float(free) / 1024.0 ** 3:.3f} GiB currently free.')
     n, nrhs = a.shape[0], b2.shape[1]
-    a_f = np.asfortranarray(a)
-    x = np.array(b2, dtype=np.complex128, order='F', copy=True)
     info = _lib.ctypes.c_int(0)
     mode = _lib.PREC_MIXED if requested_precision() == 'mixed' else _lib.PREC_FP64
+    # a C-order matrix (with right-hand sides in either order) goes up as it is and is transposed
+    # on the device; any other layout is laid out column-major here
+    rows = a.flags.c_contiguous and not a.flags.f_contiguous
+    if rows:
+        b_in = np.ascontiguousarray(b2)
+        x = np.empty((n, nrhs), dtype=np.complex128)
+
+        def call(m):
+            return ctx.lib.grim_zgesv_rowmajor(ctx.h, n, nrhs, a.ctypes.data_as(_lib.c_void_p),
+                                               b_in.ctypes.data_as(_lib.c_void_p), x.ctypes.data_as(_lib.c_void_p), m,
+                                               _lib.ctypes.byref(info))
+    else:
+        a_f = np.asfortranarray(a)
+        x = np.empty((n, nrhs), dtype=np.complex128, order='F')
+
+        def call(m):
+            x[...] = b2
+            return ctx.lib.grim_zgesv_batched(ctx.h, n, nrhs, a_f.ctypes.data_as(_lib.c_void_p), n,
+                                              x.ctypes.data_as(_lib.c_void_p), n, m, _lib.ctypes.byref(info))
     try:
         torch.cuda.current_stream().synchronize()
-        status = ctx.lib.grim_zgesv_batched(ctx.h, n, nrhs, a_f.ctypes.data_as(_lib.c_void_p), n,
-                                            x.ctypes.data_as(_lib.c_void_p), n, mode, _lib.ctypes.byref(info))
+        status = call(mode)
         if status == _lib.GRIM_ERR_NOT_CONVERGED and mode == _lib.PREC_MIXED:
             # mixed -> double ladder (reference linalg/dense.py:74-98)
-            x[...] = b2
-            status = ctx.lib.grim_zgesv_batched(ctx.h, n, nrhs, a_f.ctypes.data_as(_lib.c_void_p), n,
-                                                x.ctypes.data_as(_lib.c_void_p), n, _lib.PREC_FP64,
-                                                _lib.ctypes.byref(info))
-        _lib.check(status, 'grim_zgesv_batched')
+            status = call(_lib.PREC_FP64)
+        _lib.check(status, 'grim_zgesv')
     except _lib.GrimMemoryError as exc:
         raise MemoryError(str(exc)) from exc
     except _lib.GrimError as exc:
@@ -152,7 +165,10 @@ def _solve_dense_gpu(a_eval, rhs_eval):
     st = _lib.GrimSolveInfo()
     ctx.lib.grim_last_solve_info(ctx.h, _lib.ctypes.byref(st))
     _DENSE_BACKEND_LOCAL.last_info = st.as_dict()
-    sol = x[:, 0].copy() if vec else np.ascontiguousarray(x) if b.flags.c_contiguous else x
+    if vec:
+        sol = x[:, 0].copy()
+    else:  # laid out as the right-hand sides
+        sol = np.ascontiguousarray(x) if b.flags.c_contiguous else np.asfortranarray(x)
     return np.asarray(sol, dtype=np.complex128), ctx.device_name
 
 

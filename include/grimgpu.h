@@ -348,6 +348,12 @@ int ghost_far_block(int64_t mb, int64_t nb, int q, int width, const double *obs_
                     const uint8_t *far, int obs_normal_deriv, int want_s, int want_k, int mirrored, double k_re,
                     double k_im, int intervals, const double *bounds, int degree, const double *coeff, double *acc_s,
                     double *acc_k, double *acc_kt);
+/* ghost_far_block with accumulators that are only written: sums from zero, nothing copied in. */
+int grim_far_block_fresh(int64_t mb, int64_t nb, int q, int width, const double *obs_pts, const double *src_pts,
+                    const double *qw, const double *phi, const double *obs_norm, const double *src_norm,
+                    const uint8_t *far, int obs_normal_deriv, int want_s, int want_k, int mirrored, double k_re,
+                    double k_im, int intervals, const double *bounds, int degree, const double *coeff, double *acc_s,
+                    double *acc_k, double *acc_kt);
 /* grim_far_block: the same on DEVICE pointers, on the handle's stream (blocks until done). */
 int grim_far_block(grim_handle_t h, int64_t mb, int64_t nb, int q, int width, const double *obs_pts,
                    const double *src_pts, const double *qw, const double *phi, const double *obs_norm,
@@ -360,6 +366,10 @@ int grim_far_block(grim_handle_t h, int64_t mb, int64_t nb, int q, int width, co
  * Copies host -> device, solves, copies device -> host; synchronous. */
 int grim_zgesv_batched(grim_handle_t h, int n, int nrhs, const double *A, int lda, double *B, int ldb,
                        int precision_mode, int *info);
+/* The same for row-major (C-order, contiguous) host arrays A (n x n), B and X (n x nrhs); B is
+ * kept, the solution goes to X. */
+int grim_zgesv_rowmajor(grim_handle_t h, int n, int nrhs, const double *A, const double *B, double *X,
+                        int precision_mode, int *info);
 int grim_last_solve_info(grim_handle_t h, grim_solve_info *out);
 
 /* ---- body of revolution (PEC EFIE / MFIE / CFIE per azimuthal mode) ----------------

@@ -1,0 +1,64 @@
+"""Host-buffer entry points around the sizes where their copies change: below 2 MiB one plain
+copy, above it 1 MiB chunks through the handle's pinned slots on several threads; row-major
+systems are transposed on the device."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip('torch')
+
+
+@pytest.mark.parametrize('n, nrhs', [(1, 1), (33, 5), (361, 1), (363, 40), (600, 129)])
+@pytest.mark.parametrize('layout', ['C', 'F', 'strided'])
+def test_dense_hook_takes_every_layout(n, nrhs, layout):
+    from grim_20261007_b200.twod.solver import _solve_dense_gpu
+    rng = np.random.default_rng(n)
+
+    def lay(v):
+        if layout == 'strided':
+            out = np.zeros((2 * v.shape[0], 2 * v.shape[1]), complex)[::2, ::2]
+            out[...] = v
+            return out
+        return np.array(v, order=layout)
+
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * n ** 0.5 * np.eye(n)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    al, bl = lay(a), lay(b)
+    x, _name = _solve_dense_gpu(al, bl)
+    res = np.max(np.abs(a @ x - b)) / (np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x)))
+    assert res < 1e-14
+    assert np.array_equal(al, a) and np.array_equal(bl, b)  # the inputs are borrowed
+    assert x.flags.c_contiguous if bl.flags.c_contiguous else x.flags.f_contiguous
+    v, _name = _solve_dense_gpu(al, np.ascontiguousarray(b[:, 0]))
+    assert v.shape == (n,) and np.max(np.abs(v - x[:, 0])) <= 1e-13 * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize('rows, cols', [(3, 2), (130, 131), (181, 182), (300, 257)])
+def test_far_block_from_zero_equals_accumulating(rows, cols):
+    """Fresh accumulators equal sums into zeros; sums into other values keep them."""
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.twod import farblock
+    rng = np.random.default_rng(rows)
+    q, k = 5, 20.0
+    x, w = np.polynomial.legendre.leggauss(q)
+    s = np.linspace(0.0, 0.05, q)
+    obs = np.ascontiguousarray(np.stack([np.arange(rows)[:, None] * 0.06 + s, 0.01 * np.ones((rows, q))], -1))
+    src = np.ascontiguousarray(np.stack([np.arange(cols)[:, None] * 0.06 + s, np.full((cols, q), 1.0)], -1))
+    phi = np.ascontiguousarray(np.stack([(1 - x) / 2, (1 + x) / 2], -1))
+    qw = np.ascontiguousarray(w / 2)
+    on, sn = np.tile([0.0, 1.0], (rows, 1)), np.tile([0.6, 0.8], (cols, 1))
+    far = (rng.uniform(size=(rows, cols)) < 0.8).astype(np.uint8)
+    table = farblock.KernelTable(k, 25.0)
+    got = farblock.far_block(table, k, obs, src, qw, phi, on, sn, far, 1, True, True, True)
+    start = [rng.standard_normal((4, rows, cols)) + 1j * rng.standard_normal((4, rows, cols)) for _ in range(3)]
+    acc = [v.copy() for v in start]
+    coeff = np.ascontiguousarray(table.normalized_power)
+    lib = _lib.load()
+    assert lib.ghost_far_block(rows, cols, q, 2, obs.ctypes.data, src.ctypes.data, qw.ctypes.data, phi.ctypes.data,
+                               on.ctypes.data, sn.ctypes.data, far.ctypes.data, 1, 1, 1, 1, k, 0.0,
+                               len(table.bounds) - 1, table.bounds.ctypes.data, coeff.shape[1] - 1, coeff.ctypes.data,
+                               *(v.ctypes.data for v in acc)) == 0
+    for g, a, s0 in zip(got, acc, start):
+        assert np.all(g[:, far == 0] == 0)
+        assert np.array_equal(a[:, far == 0], s0[:, far == 0])
+        assert np.max(np.abs(a - s0 - g)) <= 1e-15 * np.max(np.abs(s0)) * 4
