@@ -513,19 +513,37 @@ extern "C" int grim_gal_farfield(grim_handle_t h, int ne, const double *elem, co
 // ============================================================== GEMM launcher
 static int tc_enabled();
 
+template <bool NEG, bool BETA, int TM, int TN>
+static int dmma_gemm_tile(grim_context *h, int M, int N, int K, const double2 *A, int64_t lda, const double2 *B,
+                          int64_t ldb, double2 *C, int64_t ldc) {
+    static PerDeviceOnce attr;
+    if (attr.needed()) {
+        GRIM_CHECK_CUDA(cudaFuncSetAttribute(k_gemm_dmma<NEG, BETA, TM, TN>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, dm_smem(TM, TN)));
+        attr.mark();
+    }
+    dim3 grid(ceil_div(M, 16 * TM), ceil_div(N, 16 * TN));
+    k_gemm_dmma<NEG, BETA, TM, TN><<<grid, DM_THREADS, dm_smem(TM, TN), h->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
+    GRIM_CHECK_LAUNCH_W(h, "k_gemm_dmma", 8.0 * M * N * K, 16.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
+    return GRIM_OK;
+}
+
+// The tile shape with the least work on the fullest SM: tiles per SM (rounded up) times tile
+// area, the smaller shapes' area raised by what they lose in a full wave (their fragment
+// loads serve fewer MMAs).  A 64 x 64 tile of K = 64 takes 12 us of one SM whatever the
+// others do: a 1000 x 64 update on the panel chain ran on 16 of 148 SMs.  The sums of an
+// element do not depend on the shape.
 template <bool NEG, bool BETA>
 static int dmma_gemm(grim_context *h, int M, int N, int K, const double2 *A, int64_t lda, const double2 *B,
                      int64_t ldb, double2 *C, int64_t ldc) {
-    static PerDeviceOnce attr;
-    if (attr.needed()) {
-        GRIM_CHECK_CUDA(
-            cudaFuncSetAttribute(k_gemm_dmma<NEG, BETA>, cudaFuncAttributeMaxDynamicSharedMemorySize, DM_SMEM_BYTES));
-        attr.mark();
-    }
-    dim3 grid(ceil_div(M, DM_BM), ceil_div(N, DM_BN));
-    k_gemm_dmma<NEG, BETA><<<grid, DM_THREADS, DM_SMEM_BYTES, h->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
-    GRIM_CHECK_LAUNCH_W(h, "k_gemm_dmma", 8.0 * M * N * K, 16.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
-    return GRIM_OK;
+    auto load = [&](int bm, int bn, double loss) {
+        const int64_t tiles = (int64_t)ceil_div(M, bm) * ceil_div(N, bn);
+        return (double)((tiles + h->sm_count - 1) / h->sm_count) * bm * bn * loss;
+    };
+    const double l44 = load(64, 64, 1.0), l42 = load(64, 32, 1.07), l22 = load(32, 32, 1.18);
+    if (l44 <= l42 && l44 <= l22) return dmma_gemm_tile<NEG, BETA, 4, 4>(h, M, N, K, A, lda, B, ldb, C, ldc);
+    if (l42 <= l22) return dmma_gemm_tile<NEG, BETA, 4, 2>(h, M, N, K, A, lda, B, ldb, C, ldc);
+    return dmma_gemm_tile<NEG, BETA, 2, 2>(h, M, N, K, A, lda, B, ldb, C, ldc);
 }
 
 // C = (BETA ? C : 0) + (NEG ? -1 : 1) A B.  Complex128 throughout: FP64 tensor cores
