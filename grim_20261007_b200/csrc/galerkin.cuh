@@ -786,6 +786,22 @@ __device__ __forceinline__ int gal_far_order(double kl_max, double ratio_min, in
 
 #define GAL_MAX_Q 16
 
+// Smallest Gauss order whose rule equals the exact integral to 1e-16 of the integral of the
+// integrand's magnitude, for g and H1/x against the linear and quadratic weights of one
+// element: |k| L <= kl_max, the other point as near as centre-distance ratio ratio_min lets an
+// element end come, the worst of five directions.  From 34-digit evaluations; the first term
+// is the 1/r growth towards the element, the second the oscillation along it.  A higher order
+// returns the same sums to rounding, so larger floors stop here (GAL_MAX_Q past kl_max = 3):
+// N = 4099 TE with a floor of 16 takes 5.5 ms instead of 16.0, N = 2048 with one of 8 1.31
+// instead of 1.42.
+__device__ __forceinline__ int gal_converged_order(double kl_max, double ratio_min) {
+    const int qr = ratio_min < 4.0 ? 10 : ratio_min < 5.0 ? 9 : ratio_min < 8.0 ? 8 : ratio_min < 14.0 ? 7
+                 : ratio_min < 30.0 ? 6 : 5;
+    const int qk = kl_max <= 0.15 ? 5 : kl_max <= 0.45 ? 6 : kl_max <= 1.0 ? 7 : kl_max <= 1.75 ? 8
+                 : kl_max <= 2.0 ? 9 : kl_max <= 3.0 ? 10 : GAL_MAX_Q;
+    return max(qr, qk);
+}
+
 // Gauss order of one 32 x 32 tile from its worst far pair, the same in every thread; 0 when
 // the tile has no far pair.
 __device__ __forceinline__ int gal_tile_order(int ne, int e0, int f0, const GalElem *so, const GalElem *ss,
@@ -816,13 +832,15 @@ __device__ __forceinline__ int gal_tile_order(int ne, int e0, int f0, const GalE
         lmax = fmax(lmax, red_l[w]);
     }
     if (!(rmin < INFINITY)) return 0;
-    return min(GAL_MAX_Q, max(min_order, gal_far_order(fabs(k) * lmax, rmin, 8)));
+    const double kl = fabs(k) * lmax;
+    return min(gal_converged_order(kl, rmin), min(GAL_MAX_Q, max(min_order, gal_far_order(kl, rmin, 8))));
 }
 
 // Far pairs of the 32 x 32 tiles of the upper tile triangle (rows ti <= cols tj; pairs e < f
 // only on diagonal tiles), gridDim.z CTAs per tile.  One set of Hankel evaluations per pair
 // gives both orientations: E[e][f] and E[f][e].  min_order: the floor on the tile order (the
-// TE rows' W rule: 8, or 16 outside its calibration; 0 for TM).
+// TE rows' W rule: 8, or 16 outside its calibration; 0 for TM), kept to rounding
+// (gal_converged_order).
 //
 // Bound by the FP64 pipe: about 85 FP64 operations a point.  r . n_s does not depend on the
 // point of the (straight) source element and r . n_o not on the observation point, so the

@@ -143,7 +143,8 @@ int grim_farfield2d(grim_handle_t h, int n, const double *geom, int nang, const 
  *   by its own CTA.
  * grim_gal_fill writes the n x n node matrix: TM (pol 0) S + gamma (D + M/2), TE (pol 1)
  * K' - M/2 - gamma W, gamma = 1/(j k).  far_min_order: floor on the far Gauss order (the
- * TE rows' W rule: 8, or 16 outside its calibration; 0 for TM).  Near pairs in FP64;
+ * TE rows' W rule: 8, or 16 outside its calibration; 0 for TM); a tile whose sums a lower
+ * order already gives to rounding (1e-16 of the kernel) takes that one.  Near pairs in FP64;
  * out_complex64 stores Z as complex64.  An adaptive pair that did not converge or a
  * failed self series sets a flag that grim_gal_status returns (and clears; synchronises).
  * grim_gal_rhs: B[:, a] = TM -load, TE -(normal-derivative load) of the plane wave

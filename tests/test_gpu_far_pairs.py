@@ -18,14 +18,14 @@ def _ring(count):
     return np.stack([np.cos(theta), 0.8 * np.sin(theta)], axis=1)
 
 
-def _far_entries(drawn, k, pol, rows, cols):
-    """Node entries (rows, cols) whose four element pairs are all far, by a 12-point rule."""
+def _far_entries(drawn, k, pol, rows, cols, order=12):
+    """Node entries (rows, cols) whose four element pairs are all far, by a rule of `order` points."""
     n = len(drawn)
     a = drawn[(-np.arange(n)) % n]
     b = np.roll(a, -1, axis=0)
     length = np.hypot(*(b - a).T)
     nrm = np.stack([-(b - a)[:, 1], (b - a)[:, 0]], axis=1) / length[:, None]
-    x, w = np.polynomial.legendre.leggauss(12)
+    x, w = np.polynomial.legendre.leggauss(order)
     x, w = 0.5 * (x + 1.0), 0.5 * w
     hat = np.stack([1.0 - x, x])
     out = np.zeros(len(rows), complex)
@@ -66,3 +66,34 @@ def test_far_entries_equal_plain_quadrature(n, kl, pol):
     cols = (rows + gap) % n
     ref = _far_entries(drawn, k, pol, rows, cols)
     assert np.max(np.abs(z[rows, cols] - ref)) <= 1e-12 * np.max(np.abs(z))
+
+
+@pytest.mark.parametrize('kl', [0.02, 0.16, 0.46, 0.9, 1.4, 1.9, 2.6])
+@pytest.mark.parametrize('floor', [8, 16])
+@pytest.mark.parametrize('pol', ['TM', 'TE'])
+def test_converged_orders_hold_every_floor(kl, floor, pol, monkeypatch):
+    """A floor above the converged order changes nothing but rounding: entries against a 16-point
+    rule over neighbouring tiles (ratios from 8) to far ones, elements of 1 : 3 lengths."""
+    from grim_20261007_b200.device import to_host_matrix
+    from grim_20261007_b200.twod.galerkin import GalerkinBody
+    monkeypatch.setattr(GalerkinBody, 'far_min_order', lambda self, k, p: floor if p == 'TE' else 0)
+    n = 400
+    theta = -2.0 * np.pi * (np.arange(n) / n)
+    theta = theta + 0.5 * np.sin(theta)
+    drawn = np.stack([np.cos(theta), 0.8 * np.sin(theta)], axis=1)
+    length = np.hypot(*(np.roll(drawn, -1, axis=0) - drawn).T)
+    k = kl / length.max()
+    z = to_host_matrix(GalerkinBody([drawn]).fill_matrix(k, pol))
+    rows = np.arange(n).repeat(12)
+    cols = (rows + np.tile([40, 47, 64, 90, 111, 150, 200, 260, 290, 333, 350, 360], n)) % n
+    pts = drawn[(-np.arange(n)) % n]
+    dist = np.hypot(*(pts[rows] - pts[cols]).T)
+    sel = dist >= 12.0 * length.max()  # TM keeps the reference's lower orders nearer in
+    rows, cols, dist = rows[sel], cols[sel], dist[sel]
+    ref = _far_entries(drawn, k, pol, rows, cols, order=16)
+    # the four element sums of an entry: kernel values carry a few ulp and the phase k r its own
+    g = 0.25 * np.hypot(special.j0(k * dist), special.y0(k * dist))
+    scale = g * (4.0 / k + 4.0 * length.max() + 4.0 * length.max() ** 2)
+    eps = np.finfo(float).eps
+    order_error = 2e-11 if pol == 'TM' else 0.0  # 5- to 8-point rules of the TM table
+    assert np.all(np.abs(z[rows, cols] - ref) <= (8.0 * eps * (8.0 + k * dist) + order_error) * scale)
