@@ -144,8 +144,9 @@ struct grim_context {
     // error flag of the tensor-core kernels (device int, zeroed at first use)
     int *tc_err = nullptr;
     // factorization look-ahead: a high-priority stream for the panel chain, a low-priority
-    // one for the wide trailing updates, and the events that order them (created lazily)
-    cudaStream_t chain = nullptr, bulk = nullptr;
+    // one for the wide trailing updates, another for the right-hand sides' forward elimination,
+    // and the events that order them (created lazily)
+    cudaStream_t chain = nullptr, bulk = nullptr, forward = nullptr;
     std::vector<cudaEvent_t> events;
     // tile-shape overrides set by the autotuner (0 = built-in rule)
     int tune_solve_bn = 0;  // output-tile width of the right-hand-side GEMMs (64 or 128)

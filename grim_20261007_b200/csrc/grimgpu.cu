@@ -203,9 +203,11 @@ extern "C" int grim_destroy(grim_handle_t h) {
     }
     if (h->chain) cudaStreamSynchronize(h->chain);
     if (h->bulk) cudaStreamSynchronize(h->bulk);
+    if (h->forward) cudaStreamSynchronize(h->forward);
     for (cudaEvent_t e : h->events) cudaEventDestroy(e);
     if (h->chain) cudaStreamDestroy(h->chain);
     if (h->bulk) cudaStreamDestroy(h->bulk);
+    if (h->forward) cudaStreamDestroy(h->forward);
     if (h->grp_exec) cudaGraphExecDestroy(h->grp_exec);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     delete h;
@@ -755,6 +757,7 @@ static int lookahead_streams(grim_context *h, int nevents) {
         GRIM_CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->chain, cudaStreamNonBlocking, greatest));
         GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->bulk, cudaStreamNonBlocking, least));
+        GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->forward, cudaStreamNonBlocking, least));
     }
     while ((int)h->events.size() < nevents) {
         cudaEvent_t e;
@@ -983,11 +986,38 @@ static int tslu_launch(grim_context *h, int n, C *A, int64_t lda, int p, int j, 
 // update of panel p is still running; panel p+1's solve waits for that update (its U12
 // reads the updated columns).  With per-launch profiling on, everything runs on the
 // handle's stream in order.
+// fwd (complex128, partial or tournament pivoting): right-hand sides whose row interchanges and
+// forward elimination run beside the panel chain, a launch per TRS_FWD_PANELS panels; on
+// return fwd->done says that L X = P B is solved (as on an error or an exact zero pivot: B is
+// overwritten).  Left to getrs when profiling per launch (one stream: nothing would overlap).
 // defer: return without reading the info / pivoted-panel flags on the host (no host
 // synchronisation: the caller queues its solves behind the factorization and reads them
 // later with getrf_read_flags); *info_host is then 0.
+struct RhsForward {
+    double2 *B;
+    int64_t ldb;
+    int nrhs;
+    bool done = false;
+};
+
+static int forward_strip(grim_context *h, int n, const RhsForward &f, const double2 *LU, int64_t lda, int p0, int p1,
+                         const int *moves_all) {
+    static PerDeviceOnce attr;
+    if (attr.needed()) {
+        GRIM_CHECK_CUDA(
+            cudaFuncSetAttribute(k_forward_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRS_FWD_SMEM));
+        attr.mark();
+    }
+    k_forward_strip<<<ceil_div(f.nrhs, TRS_COLS), TRS_FWD_THREADS, TRS_FWD_SMEM, h->forward>>>(
+        n, f.nrhs, LU, lda, f.B, f.ldb, p0, p1, moves_all);
+    const int j = p0 * NB, cols = std::min(n, p1 * NB) - j;
+    GRIM_CHECK_LAUNCH_W(h, "k_forward_strip", 8.0 * (n - j - 0.5 * cols) * cols * f.nrhs, 16.0 * (n - j) * cols);
+    return GRIM_OK;
+}
+
 template <typename C>
-static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int *info_host, bool defer = false) {
+static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int *info_host, bool defer = false,
+                      RhsForward *fwd = nullptr) {
     if (!h || n <= 0 || !A || lda < n || !ipiv) return grim_fail(GRIM_ERR_ARGUMENT, "getrf: bad arguments");
     DeviceGuard g(h->device);
     GRIM_TRY(smem_opt_in<C>());
@@ -1004,12 +1034,16 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
     const bool split = !h->profiling;
     const cudaStream_t caller = h->stream;
     cudaStream_t wide = caller;
-    // events: [0] start, [1] end, then per panel "packed" (2 + p) and "wide done" (2 + npan + p)
+    const bool forward = sizeof(C) == sizeof(double2) && fwd && split && tc_enabled() &&
+                         (h->pivot_mode == GRIM_PIVOT_PARTIAL || h->pivot_mode == GRIM_PIVOT_TOURNAMENT);
+    // events: [0] start, [1] end, then per panel "packed" (2 + p) and "wide done" (2 + npan + p),
+    // and per launch of the forward elimination "panels factored"
     if (split) {
-        GRIM_TRY(lookahead_streams(h, 2 + 2 * npan));
+        GRIM_TRY(lookahead_streams(h, 2 + 2 * npan + ceil_div(npan, TRS_FWD_PANELS)));
         GRIM_CHECK_CUDA(cudaEventRecord(h->events[0], caller));
         GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->chain, h->events[0], 0));
         GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->bulk, h->events[0], 0));
+        if (forward) GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->forward, h->events[0], 0));
         h->stream = h->chain;
         wide = h->bulk;
     } else {
@@ -1017,20 +1051,21 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
     }
     int status = GRIM_OK;
     bool wide_pending = false;
-    int *moves = nullptr;
+    int *moves_all = nullptr;  // pivoted panels: the row moves of each (GEPP_MOVES_STRIDE)
     const bool tournament = h->pivot_mode == GRIM_PIVOT_TOURNAMENT;
     TsluWs tws;
     if (h->pivot_mode == GRIM_PIVOT_PARTIAL || tournament) {
         void *pm = nullptr;
-        GRIM_TRY(grim_workspace(h, "gepp_moves", (1 + 2 * GEPP_MAX_MOVES) * sizeof(int), &pm));
-        moves = (int *)pm;
+        GRIM_TRY(grim_workspace(h, "lu_moves_all", (size_t)npan * GEPP_MOVES_STRIDE * sizeof(int), &pm));
+        moves_all = (int *)pm;
         if (tournament) GRIM_TRY(tslu_workspace<C>(h, n, &tws));
     }
-    for (int p = 0; p < npan && status == GRIM_OK && moves; ++p) {
+    for (int p = 0; p < npan && status == GRIM_OK && moves_all; ++p) {
         // partial pivoting: the panel on a cluster, then the trailing columns' row moves and
         // U12, then the trailing update (the same look-ahead as below)
         const int j = p * NB, nbj = std::min(NB, n - j);
         const int rest = n - j - nbj;
+        int *moves = moves_all + (size_t)p * GEPP_MOVES_STRIDE;
         PanelPack pk;
         const bool prepack = sizeof(C) == sizeof(float2) && tc_enabled() && nbj == NB && rest > 0;
         if (prepack) {
@@ -1047,6 +1082,18 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
         status = tournament ? tslu_launch<C>(h, n, A, lda, p, j, nbj, ipiv, d_info, swapped + p, moves, pk, tws)
                             : gepp_launch<C>(h, n, A, lda, j, nbj, ipiv, d_info, swapped + p, moves, pk);
         if (status != GRIM_OK) break;
+        if constexpr (sizeof(C) == sizeof(double2)) {
+            if (forward && ((p + 1) % TRS_FWD_PANELS == 0 || p == npan - 1)) {
+                const int q = p / TRS_FWD_PANELS;
+                const cudaEvent_t factored = h->events[2 + 2 * npan + q];
+                status = grim_cuda_status(cudaEventRecord(factored, h->stream), "cudaEventRecord");
+                if (status == GRIM_OK)
+                    status = grim_cuda_status(cudaStreamWaitEvent(h->forward, factored, 0), "cudaStreamWaitEvent");
+                if (status == GRIM_OK)
+                    status = forward_strip(h, n, *fwd, A, lda, q * TRS_FWD_PANELS, p + 1, moves_all);
+                if (status != GRIM_OK) break;
+            }
+        }
         if (wide_pending) {
             GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0));
             wide_pending = false;
@@ -1066,7 +1113,7 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
             }
         }
     }
-    for (int p = 0; p < npan && status == GRIM_OK && !moves; ++p) {
+    for (int p = 0; p < npan && status == GRIM_OK && !moves_all; ++p) {
         const int j = p * NB, nbj = std::min(NB, n - j);
         k_diag_lu<C><<<1, 256, 0, h->stream>>>(n, A, lda, j, nbj, bcol, cert + p, ipiv);
         status = grim_launch_status(h, kname("k_diag_lu", sizeof(C)), 8.0 * nbj * nbj * nbj / 3.0, 0);
@@ -1111,21 +1158,19 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
             status = grim_launch_status(h, kname("k_panel_last", sizeof(C)), 0, 0);
         }
     }
-    if (status == GRIM_OK && moves && (size_t)n * sizeof(C) <= GEPP_MOVES_SMEM_MAX && n > NB) {
-        // partial pivoting: every panel's row moves, then each factored column takes those of
-        // the panels after it (one CTA per column, in shared memory)
-        void *pm = nullptr;
-        status = grim_workspace(h, "lu_moves_all", (size_t)npan * GEPP_MOVES_STRIDE * sizeof(int), &pm);
-        if (status == GRIM_OK) {
-            k_ipiv_moves<<<ceil_div(npan, 4), 128, 0, h->stream>>>(n, ipiv, (int *)pm);
-            status = grim_launch_status(h, "k_ipiv_moves", 0, 0);
-        }
-        if (status == GRIM_OK) {
-            const int ncols = (npan - 1) * NB;
-            k_apply_moves<C><<<ncols, 256, (size_t)n * sizeof(C), h->stream>>>(n, A, lda, 0, 1, (const int *)pm,
-                                                                                nullptr);
-            status = grim_launch_status(h, kname("k_apply_moves_left", sizeof(C)), 0, 0);
-        }
+    if (forward) {
+        // the left interchanges move the rows of L that the forward elimination reads; the
+        // caller's stream waits for it through the chain, whatever happened above
+        cudaEventRecord(h->events[1], h->forward);
+        cudaStreamWaitEvent(h->chain, h->events[1], 0);
+        fwd->done = true;
+    }
+    if (status == GRIM_OK && moves_all && (size_t)n * sizeof(C) <= GEPP_MOVES_SMEM_MAX && n > NB) {
+        // partial pivoting: each factored column takes the row moves of the panels after its own
+        // (one CTA per column, in shared memory)
+        const int ncols = (npan - 1) * NB;
+        k_apply_moves<C><<<ncols, 256, (size_t)n * sizeof(C), h->stream>>>(n, A, lda, 0, 1, moves_all, nullptr);
+        status = grim_launch_status(h, kname("k_apply_moves_left", sizeof(C)), 0, 0);
     } else if (status == GRIM_OK) {
         k_laswp_left<C><<<ceil_div(n, 128), 128, 0, h->stream>>>(n, A, lda, NB, swapped, ipiv);
         status = grim_launch_status(h, kname("k_laswp_left", sizeof(C)), 0, 0);
@@ -1231,6 +1276,25 @@ static int trsolve_strip(grim_context *h, int n, int nrhs, const double2 *LU, in
     return GRIM_OK;
 }
 
+// B <- U^-1 B.
+template <typename C>
+static int getrs_upper(grim_context *h, int n, int nrhs, const C *LU, int64_t lda, C *B, int64_t ldb) {
+    const int npan = ceil_div(n, NB);
+    const size_t tri = (size_t)(NB * NBP + NB) * sizeof(C);
+    if constexpr (sizeof(C) == sizeof(double2)) {
+        if (trsolve_wanted(n, nrhs)) return trsolve_strip<true>(h, n, nrhs, LU, lda, B, ldb);
+    }
+    const int ctiles = ceil_div(nrhs, TRSM_COLS);
+    for (int p = npan - 1; p >= 0; --p) {
+        const int j = p * NB, nbj = std::min(NB, n - j);
+        k_trsm_diag<C, true><<<ctiles, 4 * TRSM_COLS, tri, h->stream>>>(nrhs, LU, lda, B, ldb, j, nbj, 0, 0);
+        GRIM_CHECK_LAUNCH_W(h, kname("k_trsm_diag", sizeof(C)), 4.0 * nbj * nbj * nrhs, 0);
+        if (j > 0)
+            GRIM_TRY((gemm_sub<C>(h, j, nrhs, nbj, LU + (int64_t)j * lda, lda, B + j, ldb, B, ldb)));
+    }
+    return GRIM_OK;
+}
+
 template <typename C>
 static int getrs_apply(grim_context *h, int n, int nrhs, const C *LU, int64_t lda, const int *ipiv, const int *ident,
                        C *B, int64_t ldb) {
@@ -1240,7 +1304,7 @@ static int getrs_apply(grim_context *h, int n, int nrhs, const C *LU, int64_t ld
     if constexpr (sizeof(C) == sizeof(double2)) {
         if (trsolve_wanted(n, nrhs)) {
             GRIM_TRY((trsolve_strip<false>(h, n, nrhs, LU, lda, B, ldb)));
-            return trsolve_strip<true>(h, n, nrhs, LU, lda, B, ldb);
+            return getrs_upper<C>(h, n, nrhs, LU, lda, B, ldb);
         }
     }
     const int ctiles = ceil_div(nrhs, TRSM_COLS);
@@ -1253,14 +1317,7 @@ static int getrs_apply(grim_context *h, int n, int nrhs, const C *LU, int64_t ld
             GRIM_TRY((gemm_sub<C>(h, below, nrhs, nbj, LU + (int64_t)j * lda + j + nbj, lda, B + j, ldb,
                                                   B + j + nbj, ldb)));
     }
-    for (int p = npan - 1; p >= 0; --p) {
-        const int j = p * NB, nbj = std::min(NB, n - j);
-        k_trsm_diag<C, true><<<ctiles, 4 * TRSM_COLS, tri, h->stream>>>(nrhs, LU, lda, B, ldb, j, nbj, 0, 0);
-        GRIM_CHECK_LAUNCH_W(h, kname("k_trsm_diag", sizeof(C)), 4.0 * nbj * nbj * nrhs, 0);
-        if (j > 0)
-            GRIM_TRY((gemm_sub<C>(h, j, nrhs, nbj, LU + (int64_t)j * lda, lda, B + j, ldb, B, ldb)));
-    }
-    return GRIM_OK;
+    return getrs_upper<C>(h, n, nrhs, LU, lda, B, ldb);
 }
 
 template <typename C>
@@ -1879,8 +1936,23 @@ extern "C" int grim_zgesv_mixed(grim_handle_t h, int n, int nrhs, const void *A,
         double2 *lu = (double2 *)plu;
         GRIM_CHECK_CUDA(cudaMemcpy2DAsync(lu, n * sizeof(double2), A, lda * sizeof(double2), n * sizeof(double2), n,
                                           cudaMemcpyDeviceToDevice, h->stream));
+        // the forward elimination beside the factorization overwrites B: kept for a singular A
+        // (no room for the copy: B waits for getrs)
+        void *pB0 = nullptr;
+        const size_t row = n * sizeof(double2);
+        const bool kept = grim_workspace(h, "gd_B0", row * nrhs, &pB0) == GRIM_OK;
+        if (kept)
+            GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pB0, row, B, ldb * sizeof(double2), row, nrhs, cudaMemcpyDeviceToDevice,
+                                              h->stream));
+        else
+            cudaGetLastError();
+        RhsForward fwd{(double2 *)B, ldb, nrhs};
         StreamTimer tf(h->stream);
-        GRIM_TRY(getrf_impl<double2>(h, n, lu, n, ipiv, &linfo));
+        const int fs = getrf_impl<double2>(h, n, lu, n, ipiv, &linfo, false, kept ? &fwd : nullptr);
+        if ((fs != GRIM_OK || linfo > 0) && fwd.done)
+            GRIM_CHECK_CUDA(cudaMemcpy2DAsync(B, ldb * sizeof(double2), pB0, row, row, nrhs, cudaMemcpyDeviceToDevice,
+                                              h->stream));
+        GRIM_TRY(fs);
         st.ms_factor = tf.stop_ms();
         st.pivoted_panels = h->last.pivoted_panels;
         if (linfo > 0) {
@@ -1890,7 +1962,10 @@ extern "C" int grim_zgesv_mixed(grim_handle_t h, int n, int nrhs, const void *A,
             return grim_fail(GRIM_ERR_SINGULAR, "grim_zgesv_mixed: matrix is exactly singular");
         }
         StreamTimer ts(h->stream);
-        GRIM_TRY(getrs_impl<double2>(h, n, nrhs, lu, n, ipiv, (double2 *)B, ldb));
+        if (fwd.done)
+            GRIM_TRY(getrs_upper<double2>(h, n, nrhs, lu, n, (double2 *)B, ldb));
+        else
+            GRIM_TRY(getrs_impl<double2>(h, n, nrhs, lu, n, ipiv, (double2 *)B, ldb));
         st.ms_solve = ts.stop_ms();
         st.backward_error = -1.0;
     } else {
@@ -1981,8 +2056,12 @@ extern "C" int grim_zgesv_guarded(grim_handle_t h, int n, int nrhs, const void *
         int linfo = 0;
         GRIM_CHECK_CUDA(cudaMemcpy2DAsync(lu, n * sizeof(double2), A, lda * sizeof(double2), n * sizeof(double2), n,
                                           cudaMemcpyDeviceToDevice, h->stream));
+        if (attempt == 1)
+            GRIM_CHECK_CUDA(cudaMemcpy2DAsync(X, ldb * sizeof(double2), B0, n * sizeof(double2), n * sizeof(double2),
+                                              nrhs, cudaMemcpyDeviceToDevice, h->stream));
         StreamTimer tf(h->stream);
-        status = getrf_impl<double2>(h, n, lu, n, ipiv, &linfo);
+        RhsForward fwd{X, ldb, nrhs};
+        status = getrf_impl<double2>(h, n, lu, n, ipiv, &linfo, false, &fwd);
         h->pivot_mode = keep;
         if (status != GRIM_OK) break;
         st.ms_factor += tf.stop_ms();
@@ -1993,13 +2072,16 @@ extern "C" int grim_zgesv_guarded(grim_handle_t h, int n, int nrhs, const void *
             st.info = linfo;
             h->last = st;
             if (info) *info = linfo;
+            if (fwd.done)
+                GRIM_CHECK_CUDA(cudaMemcpy2DAsync(X, ldb * sizeof(double2), B0, n * sizeof(double2),
+                                                  n * sizeof(double2), nrhs, cudaMemcpyDeviceToDevice, h->stream));
             return grim_fail(GRIM_ERR_SINGULAR, "grim_zgesv_guarded: matrix is exactly singular");
         }
         StreamTimer ts(h->stream);
-        if (attempt == 1)
-            GRIM_CHECK_CUDA(cudaMemcpy2DAsync(X, ldb * sizeof(double2), B0, n * sizeof(double2), n * sizeof(double2),
-                                              nrhs, cudaMemcpyDeviceToDevice, h->stream));
-        GRIM_TRY(getrs_impl<double2>(h, n, nrhs, lu, n, ipiv, X, ldb));
+        if (fwd.done)
+            GRIM_TRY(getrs_upper<double2>(h, n, nrhs, lu, n, X, ldb));
+        else
+            GRIM_TRY(getrs_impl<double2>(h, n, nrhs, lu, n, ipiv, X, ldb));
         GRIM_TRY(residual_and_berr(h, n, nrhs, (const double2 *)A, lda, X, ldb, B0, n, R, n, sc, berr_dev, nullptr,
                                    sc + 1));
         double hv = INFINITY;

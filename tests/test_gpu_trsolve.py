@@ -57,3 +57,49 @@ def test_getrs_strips_keep_columns_apart():
     keep = [c for c in range(11) if c != 3]
     assert np.array_equal(x[:, keep], clean[:, keep])
     assert not np.all(np.isfinite(x[:, 3]))
+
+
+def _solve(a, b, pivot, lda, ldb):
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.device import context, ptr
+    ctx = context()
+    n, nrhs = b.shape
+    ad = torch.zeros((n, lda), dtype=torch.complex128)
+    ad[:, :n] = torch.from_numpy(np.ascontiguousarray(a.T))
+    x = torch.full((nrhs, ldb), 7.0 - 3.0j, dtype=torch.complex128)
+    x[:, :n] = torch.from_numpy(np.ascontiguousarray(b.T))
+    ad, x = ad.cuda(), x.cuda()
+    info = ctypes.c_int(0)
+    status = ctx.lib.grim_zgesv_mixed(ctx.h, n, nrhs, ptr(ad), lda, None, 0, ptr(x), ldb, _lib.PREC_FP64 | pivot,
+                                      1e-10, 0, ctypes.byref(info), None)
+    out = x.cpu().numpy()
+    assert np.all(out[:, n:] == 7.0 - 3.0j)
+    return status, info.value, out[:, :n].T
+
+
+@pytest.mark.parametrize('n', [1, 63, 64, 65, 255, 256, 257, 321, 513])
+@pytest.mark.parametrize('nrhs', [1, 8, 9, 33])
+@pytest.mark.parametrize('mode', ['PREC_PARTIAL_PIVOT', 'PREC_TOURNAMENT_PIVOT'])
+def test_elimination_beside_the_factorization(n, nrhs, mode):
+    """Right-hand sides eliminated panel by panel (edges of panels and of the groups of four)."""
+    from grim_20261007_b200 import _lib
+    rng = np.random.default_rng(100 * n + nrhs)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    status, info, x = _solve(a, b, getattr(_lib, mode), n + 3, n + 5)
+    assert status == 0 and info == 0
+    res = np.max(np.abs(a @ x - b), axis=0)
+    den = np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x), axis=0) + np.max(np.abs(b), axis=0)
+    assert np.max(res / den) < 1e-14
+
+
+def test_singular_matrix_leaves_the_right_hand_sides():
+    from grim_20261007_b200 import _lib
+    n = 300
+    rng = np.random.default_rng(3)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    a[:, 270] = 0.0
+    b = rng.standard_normal((n, 10)) + 1j * rng.standard_normal((n, 10))
+    status, info, x = _solve(a, b, _lib.PREC_PARTIAL_PIVOT, n, n)
+    assert status != 0 and info == 271
+    assert np.array_equal(x, b)
