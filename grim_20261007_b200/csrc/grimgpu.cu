@@ -987,7 +987,7 @@ static int tslu_launch(grim_context *h, int n, C *A, int64_t lda, int p, int j, 
 // reads the updated columns).  With per-launch profiling on, everything runs on the
 // handle's stream in order.
 // fwd (complex128, partial or tournament pivoting): right-hand sides whose row interchanges and
-// forward elimination run beside the panel chain, a launch per TRS_FWD_PANELS panels; on
+// forward elimination run beside the panel chain (k_forward_strip, one to four panels a launch); on
 // return fwd->done says that L X = P B is solved (as on an error or an exact zero pivot: B is
 // overwritten).  Left to getrs when profiling per launch (one stream: nothing would overlap).
 // defer: return without reading the info / pivoted-panel flags on the host (no host
@@ -1036,10 +1036,9 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
     cudaStream_t wide = caller;
     const bool forward = sizeof(C) == sizeof(double2) && fwd && split && tc_enabled() &&
                          (h->pivot_mode == GRIM_PIVOT_PARTIAL || h->pivot_mode == GRIM_PIVOT_TOURNAMENT);
-    // events: [0] start, [1] end, then per panel "packed" (2 + p) and "wide done" (2 + npan + p),
-    // and per launch of the forward elimination "panels factored"
+    // events: [0] start, [1] end, then per panel "packed" (2 + p) and "wide done" (2 + npan + p)
     if (split) {
-        GRIM_TRY(lookahead_streams(h, 2 + 2 * npan + ceil_div(npan, TRS_FWD_PANELS)));
+        GRIM_TRY(lookahead_streams(h, 2 + 2 * npan));
         GRIM_CHECK_CUDA(cudaEventRecord(h->events[0], caller));
         GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->chain, h->events[0], 0));
         GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->bulk, h->events[0], 0));
@@ -1060,6 +1059,7 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
         moves_all = (int *)pm;
         if (tournament) GRIM_TRY(tslu_workspace<C>(h, n, &tws));
     }
+    int fwd_next = 0, fwd_rows = 0;
     for (int p = 0; p < npan && status == GRIM_OK && moves_all; ++p) {
         // partial pivoting: the panel on a cluster, then the trailing columns' row moves and
         // U12, then the trailing update (the same look-ahead as below)
@@ -1083,16 +1083,22 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
                             : gepp_launch<C>(h, n, A, lda, j, nbj, ipiv, d_info, swapped + p, moves, pk);
         if (status != GRIM_OK) break;
         if constexpr (sizeof(C) == sizeof(double2)) {
-            if (forward && ((p + 1) % TRS_FWD_PANELS == 0 || p == npan - 1)) {
-                const int q = p / TRS_FWD_PANELS;
-                const cudaEvent_t factored = h->events[2 + 2 * npan + q];
-                status = grim_cuda_status(cudaEventRecord(factored, h->stream), "cudaEventRecord");
+            // the forward elimination by the panels before this one starts with it (at the event
+            // of the last wide update) and is issued after it: a cluster of 16 CTAs finds no room
+            // once strips hold half the SMs
+            const bool last = rest == 0, due = fwd_rows >= TRS_FWD_ROWS || p - fwd_next >= TRS_FWD_PANELS;
+            if (forward && (last || (due && rest + nbj > NB))) {
+                if (last) status = grim_cuda_status(cudaEventRecord(h->events[2 + p], h->stream), "cudaEventRecord");
                 if (status == GRIM_OK)
-                    status = grim_cuda_status(cudaStreamWaitEvent(h->forward, factored, 0), "cudaStreamWaitEvent");
-                if (status == GRIM_OK)
-                    status = forward_strip(h, n, *fwd, A, lda, q * TRS_FWD_PANELS, p + 1, moves_all);
+                    status = grim_cuda_status(
+                        cudaStreamWaitEvent(h->forward, h->events[last ? 2 + p : 2 + p - 1], 0), "cudaStreamWaitEvent");
+                const int upto = last ? npan : p;
+                if (status == GRIM_OK) status = forward_strip(h, n, *fwd, A, lda, fwd_next, upto, moves_all);
                 if (status != GRIM_OK) break;
+                fwd_next = upto;
+                fwd_rows = 0;
             }
+            fwd_rows += rest;
         }
         if (wide_pending) {
             GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0));

@@ -192,14 +192,17 @@ k_trsolve_strip(int n, int nrhs, const double2 *__restrict__ LU, int64_t lda, do
 // right-looking, because the rows of L still move: per panel the row moves, the substitution,
 // and W -= L X on all rows below, a warp eight rows of all 64 columns at a time.
 //
-// The panel chain of the factorization leaves most SMs idle; this runs in its shadow, a launch
-// per TRS_FWD_PANELS panels, so that of the forward substitution (N = 2048, 720 columns 0.98 ms,
-// N = 1024, 361 0.28 ms) only the last launch is waited for.  256 threads and half the
-// registers of an SM: the chain's short kernels fit beside it.  Whole solves: N = 333, 19
-// columns 1.16 -> 1.08 ms (1.09 with two panels a launch, 1.13 with eight), N = 2048, 720
-// columns 9.49 -> 9.05 ms.
+// The panel chain of the factorization leaves most SMs idle; this runs in its shadow, so that of
+// the forward substitution (N = 2048, 720 columns 0.98 ms, N = 1024, 361 0.28 ms) only the last
+// launch is waited for.  A launch takes the panels of about TRS_FWD_ROWS rows of updates (at
+// 90 strips 80 us, within the 115 us of the panel that starts with it: strips still running
+// keep the next panel's 16-CTA cluster waiting, 200 us with four panels of 1900 rows a launch),
+// at most TRS_FWD_PANELS.  256 threads and half the registers of an SM: the chain's short
+// kernels fit beside it.  Whole solves: N = 333, 19 columns 1.16 -> 1.08 ms, N = 2048, 720
+// columns 9.49 -> 8.58 ms (four panels a launch from the start: 9.05).
 #define TRS_FWD_THREADS 256
 #define TRS_FWD_PANELS 4
+#define TRS_FWD_ROWS 1536
 #define TRS_FWD_LDX (NB + 4)  // eight columns' 16-byte elements in different banks
 #define TRS_FWD_SMEM ((size_t)(NB * TRS_LDT + TRS_COLS * TRS_FWD_LDX) * sizeof(double2))
 __global__ void __launch_bounds__(TRS_FWD_THREADS, 2)
