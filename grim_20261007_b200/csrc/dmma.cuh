@@ -17,10 +17,15 @@
 #define DM_BM 64
 #define DM_BN 64
 #define DM_BK 8
-#define DM_STAGES 3
 #define DM_THREADS 128
 // shared tiles padded by two complex elements per k (conflict-free fragment reads)
-__host__ __device__ constexpr int dm_smem(int tm, int tn) { return DM_STAGES * DM_BK * (16 * tm + 16 * tn + 4) * 16; }
+// Stages in flight by tile: the small ones run short K on few CTAs an SM and wait for L2 (six
+// stages and C read before the main loop: rank-64 updates of N = 2048 11.0 -> 8.3 us, of N = 333
+// 10.1 -> 7.3, 1024 x 361 x 1024 0.160 -> 0.148 ms); 64 x 64 holds two CTAs an SM with three.
+__host__ __device__ constexpr int dm_stages(int tm, int tn) { return tm * tn <= 4 ? 6 : tm * tn <= 8 ? 4 : 3; }
+__host__ __device__ constexpr int dm_smem(int tm, int tn) {
+    return dm_stages(tm, tn) * DM_BK * (16 * tm + 16 * tn + 4) * 16;
+}
 #define DM_SMEM_BYTES dm_smem(4, 4)
 
 __device__ __forceinline__ void dm_cp16(void *smem, const void *gmem, bool valid) {
@@ -39,10 +44,11 @@ template <bool NEG, bool BETA, int TM = 4, int TN = 4>
 __device__ __forceinline__ void gemm_dmma_cta(int M, int N, int K, const double2 *__restrict__ A, int64_t lda,
                                               const double2 *__restrict__ B, int64_t ldb, double2 *__restrict__ C,
                                               int64_t ldc, int m0, int n0) {
+    constexpr int STAGES = dm_stages(TM, TN);
     constexpr int BM = 16 * TM, BN = 16 * TN, LDA = BM + 2, LDB = BN + 2;
     extern __shared__ __align__(16) unsigned char dm_tiles[];
     double2 *As = reinterpret_cast<double2 *>(dm_tiles);              // [stage][k][LDA]
-    double2 *Bs = As + DM_STAGES * DM_BK * LDA;                     // [stage][k][LDB] (k-major rows of n)
+    double2 *Bs = As + STAGES * DM_BK * LDA;                     // [stage][k][LDB] (k-major rows of n)
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int g = lane >> 2, q = lane & 3;
     const int wm = (warp >> 1) * 8 * TM, wn = (warp & 1) * 8 * TN;
@@ -76,19 +82,33 @@ __device__ __forceinline__ void gemm_dmma_cta(int M, int N, int K, const double2
 #pragma unroll
         for (int j = 0; j < TN; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
 
+    // small tiles (short K, latency-bound): C arrives under the main loop
+    constexpr bool early = BETA && TM * TN <= 4;
+    double2 old[early ? TM : 1][early ? TN : 1][2];
+    if constexpr (early) {
 #pragma unroll
-    for (int s = 0; s < DM_STAGES - 1; ++s) {
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int gm = min(m0 + wm + 8 * i + g, M - 1), gn = min(n0 + wn + 8 * j + 2 * q + c, N - 1);
+                    old[i][j][c] = C[(int64_t)gn * ldc + gm];
+                }
+    }
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
         if (s < nk) load_stage(s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int kt = 0; kt < nk; ++kt) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(DM_STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();
         // prefetch stage kt + STAGES - 1 into the buffer freed by stage kt - 1
-        if (kt + DM_STAGES - 1 < nk) load_stage((kt + DM_STAGES - 1) % DM_STAGES, kt + DM_STAGES - 1);
+        if (kt + STAGES - 1 < nk) load_stage((kt + STAGES - 1) % STAGES, kt + STAGES - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const double2 *as = As + (kt % DM_STAGES) * DM_BK * LDA;
-        const double2 *bs = Bs + (kt % DM_STAGES) * DM_BK * LDB;
+        const double2 *as = As + (kt % STAGES) * DM_BK * LDA;
+        const double2 *bs = Bs + (kt % STAGES) * DM_BK * LDB;
 #pragma unroll
         for (int ks = 0; ks < DM_BK; ks += 4) {
             double ar[TM], ai[TM], nai[TM], br[TN], bi[TN];
@@ -135,7 +155,9 @@ __device__ __forceinline__ void gemm_dmma_cta(int M, int N, int K, const double2
                 }
                 double2 *p = C + (int64_t)gn * ldc + gm;
                 if (BETA) {
-                    const double2 o = *p;
+                    double2 o;
+                    if constexpr (early) o = old[i][j][c];
+                    else o = *p;
                     vr += o.x;
                     vi += o.y;
                 }
