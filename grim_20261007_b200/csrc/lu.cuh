@@ -163,6 +163,17 @@ __device__ __forceinline__ C one_c() {
 // distinct banks.
 #define NBP 65
 
+// One element from global to shared memory with cp.async (zero when not valid).
+template <typename C>
+__device__ __forceinline__ void cp_async_elem(C *smem, const C *gmem, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    const int bytes = valid ? (int)sizeof(C) : 0;
+    if constexpr (sizeof(C) == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem), "r"(bytes) : "memory");
+}
+
 template <typename C>
 __device__ __forceinline__ C shfl_xor_c(C v, int m) {
     v.x = __shfl_xor_sync(0xffffffffu, v.x, m);

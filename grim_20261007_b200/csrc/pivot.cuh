@@ -394,77 +394,114 @@ __device__ __forceinline__ int gepp_warp_argmax(unsigned long long key, unsigned
     return bal ? __ffs(bal) - 1 : -1;
 }
 
-// U12 = inv(L11) A12 of the trailing columns after the panel's row moves: one CTA per
-// blockDim.x / 4 columns (UMOVES_THREADS: 32 columns), 4 threads per column, so that the
-// 64-step substitution chains of a panel spread over about twice as many SMs as there are
-// 64-column blocks.  Each column gathers every move's source before writing any
-// destination.  complex64: also writes the trailing update's packed B operand.  Dynamic
-// smem: NB * NBP + NB elements (the diagonal block and its reciprocals).
+// L x = a (L unit lower in T, zero elsewhere) for one 64-long column vector shared by 8 lanes
+// (v[i] = row 8 i + s), right-looking: an entry, once final, is broadcast to its lanes and
+// subtracted from the later ones; after each block of eight the pending entries shift down a
+// register (the loop body stays in the instruction cache).  Blocks [b0, b0 + 4), 8 - b0 live.
+template <typename C, int B0>
+__device__ __forceinline__ void umoves_blocks(C (&v)[8], C (&x)[8], const C *T, int s) {
+    const int base = (int)(threadIdx.x & 31u) & ~7;
+#pragma unroll 1
+    for (int b = B0; b < B0 + 4; ++b) {
+#pragma unroll
+        for (int cc = 0; cc < 8; ++cc) {
+            const C xr = shfl_c(v[0], base | cc);
+            const C *col = T + (8 * b + cc) * NBP + 8 * b + s;
+            if (s > cc) cfms(v[0], xr, col[0]);
+#pragma unroll
+            for (int i = 1; i < 8 - B0; ++i)
+                if (b + i < 8) cfms(v[i], xr, col[8 * i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 7; ++i) x[i] = x[i + 1];
+        x[7] = v[0];
+#pragma unroll
+        for (int i = 0; i + 1 < 8 - B0; ++i) v[i] = v[i + 1];
+    }
+}
+
+// U12 = inv(L11) A12 of the trailing columns after the panel's row moves: 16 columns per CTA, 8
+// threads a column (a panel's substitution chains on as many SMs as there are 16-column
+// blocks; with 4 threads a column and 32 columns an SM the FP64 issue, not the chain, set the
+// time).  Between a panel and the next on the critical chain, and all latency, so the loads
+// wait on one another as little as they can: L11 comes with cp.async under the move list (one
+// read, whatever its count), and the panel's rows are read straight from where the moves take
+// them, together with the rows that leave for below it (each column gathers every source
+// before any write).  N = 2048: complex128 13.8 -> 11.3 us a panel (11.8 with 4 threads a column),
+// complex64 11.4 -> 8.9.  complex64: also writes the trailing update's packed B operand.
+// Dynamic smem: NB * NBP elements (L11).
 #define UMOVES_THREADS 128
+#define UMOVES_COLS (UMOVES_THREADS / 8)
 template <typename C>
 __global__ void __launch_bounds__(UMOVES_THREADS)
 k_panel_u_moves(int n, C *__restrict__ A, int64_t lda, int j, int nbj, const int *__restrict__ moves, PanelPack pk) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *T = reinterpret_cast<C *>(smem_raw);
-    C *rd = T + NB * NBP;
-    __shared__ int s_dst[GEPP_MAX_MOVES], s_src[GEPP_MAX_MOVES];
-    __shared__ int s_cnt;
-    const int t = threadIdx.x, s = t & 3, lane_vec = t >> 2;
-    const int cols_per_cta = (int)blockDim.x >> 2;
-    if (t == 0) s_cnt = min(moves[0], GEPP_MAX_MOVES);
+    __shared__ int s_from[NB];                 // the source of each panel row
+    __shared__ int s_dst[NB], s_src[NB];       // rows that end below the panel (at most NB)
+    __shared__ int s_below;
+    const int t = threadIdx.x, s = t & 7, lane_vec = t >> 3;
+    for (int e = t; e < NB * NB; e += UMOVES_THREADS) {
+        const int r = e % NB, c = e / NB;
+        cp_async_elem(T + c * NBP + r, A + (int64_t)(j + min(c, nbj - 1)) * lda + j + min(r, nbj - 1), c < r && r < nbj);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    static_assert(UMOVES_THREADS == GEPP_MAX_MOVES, "one move a thread");
+    const int cnt = min(moves[0], GEPP_MAX_MOVES), dst = moves[1 + t], src = moves[1 + GEPP_MAX_MOVES + t];
+    if (t < NB) s_from[t] = j + t;
+    if (t == 0) s_below = 0;
     __syncthreads();
-    const int cnt = s_cnt;
-    for (int i = t; i < cnt; i += blockDim.x) {
-        s_dst[i] = moves[1 + i];
-        s_src[i] = moves[1 + GEPP_MAX_MOVES + i];
+    if (t < cnt) {
+        if (dst < j + nbj) s_from[dst - j] = src;
+        else {
+            const int at = atomicAdd(&s_below, 1);
+            if (at < NB) {
+                s_dst[at] = dst;
+                s_src[at] = src;
+            }
+        }
     }
     __syncthreads();
-    const int col = j + nbj + cols_per_cta * blockIdx.x + lane_vec;
+    const int below = min(s_below, NB);
+    const int col = j + nbj + UMOVES_COLS * blockIdx.x + lane_vec;
     const bool ok = col < n;
-    // every source of the column is read (by its 4 threads, one warp) before any destination
-    // is written; the warp barriers stay outside the per-column condition, which differs
-    // between the lanes of a warp at the matrix edge
     C *a = A + (int64_t)col * lda;
-    C tmp[GEPP_MAX_MOVES / 4];
-    if (ok) {
+    C v[8], x[8], tmp[NB / 8];
 #pragma unroll
-        for (int q = 0; q < GEPP_MAX_MOVES / 4; ++q) {
-            const int i = 4 * q + s;
-            if (i < cnt) tmp[q] = a[s_src[i]];
-        }
+    for (int i = 0; i < 8; ++i) {
+        const int r = 8 * i + s;
+        v[i] = (ok && r < nbj) ? a[s_from[r]] : czero<C>();
     }
+#pragma unroll
+    for (int q = 0; q < NB / 8; ++q)
+        if (ok && 8 * q + s < below) tmp[q] = a[s_src[8 * q + s]];
+    // a column's 8 threads (one warp) have read all they need; the warp barrier stays outside
+    // the per-column condition, which differs between the lanes of a warp at the matrix edge
     __syncwarp();
+#pragma unroll
+    for (int q = 0; q < NB / 8; ++q)
+        if (ok && 8 * q + s < below) a[s_dst[8 * q + s]] = tmp[q];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = czero<C>();
+    umoves_blocks<C, 0>(v, x, T, s);
+    umoves_blocks<C, 4>(v, x, T, s);
     if (ok) {
 #pragma unroll
-        for (int q = 0; q < GEPP_MAX_MOVES / 4; ++q) {
-            const int i = 4 * q + s;
-            if (i < cnt) a[s_dst[i]] = tmp[q];
-        }
-    }
-    __syncwarp();
-    stage_diag(A, lda, j, nbj, T, rd);
-    C v[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int r = 4 * i + s;
-        v[i] = (ok && r < nbj) ? A[(int64_t)col * lda + j + r] : czero<C>();
-    }
-    subst_col_lower1_loop(v, T, s);
-    if (ok) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int r = 4 * i + s;
-            if (r < nbj) A[(int64_t)col * lda + j + r] = v[i];
+        for (int i = 0; i < 8; ++i) {
+            const int r = 8 * i + s;
+            if (r < nbj) A[(int64_t)col * lda + j + r] = x[i];
         }
     }
     if constexpr (sizeof(C) == sizeof(float2)) {
         if (pk.b_hi) {
-            const int nb_row = cols_per_cta * blockIdx.x + lane_vec;
+            const int nb_row = UMOVES_COLS * blockIdx.x + lane_vec;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int r = 4 * i + s;
-                pack_pair(pk.b_hi, pk.b_lo, tc_tile_offset(nb_row, 2 * r, pk.b_rows), ok ? (float)v[i].x : 0.f,
-                          ok ? (float)v[i].y : 0.f);
+            for (int i = 0; i < 8; ++i) {
+                const int r = 8 * i + s;
+                pack_pair(pk.b_hi, pk.b_lo, tc_tile_offset(nb_row, 2 * r, pk.b_rows), ok ? (float)x[i].x : 0.f,
+                          ok ? (float)x[i].y : 0.f);
             }
         }
     }
