@@ -3059,7 +3059,7 @@ extern "C" int grim_bor_excitation(grim_handle_t h, int ne, const double *nodes,
     k_bor_bessel<<<dim3(ceil_div(BOR_FAR_ORDER * ne, 128), nth), 128, 0, h->stream>>>(ne, nodes, k, m, nth, thetas_deg,
                                                                                       (double *)p_tab);
     GRIM_CHECK_LAUNCH(h, "k_bor_bessel");
-    dim3 grid(ceil_div(nred, 128), 2 * nth);
+    dim3 grid(ceil_div(nred, 128), nth);
     k_bor_excitation<<<grid, 128, 0, h->stream>>>(ne, nodes, m, nth, thetas_deg, (const double *)p_tab, far, alpha,
                                                   nred, red_full, (const double2 *)red_w, (double2 *)V, ldv);
     GRIM_CHECK_LAUNCH(h, "k_bor_excitation");
