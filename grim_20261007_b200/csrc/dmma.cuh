@@ -5,8 +5,8 @@
 // real and imaginary FP64 accumulators (64 doubles per thread at 4 x 4).  One
 // complex k-step of a tile is four real MMAs:
 //   re += Ar Br,  re += (-Ai) Bi,  im += Ar Bi,  im += Ai Br.
-// K in stages of 8 complex (two MMA k-steps), three shared-memory stages filled with
-// cp.async (16 bytes = one complex element, zero-filled outside the matrices).
+// K in stages of 8 complex (two MMA k-steps), three to six of them in shared memory, filled
+// with cp.async (16 bytes = one complex element, zero-filled outside the matrices).
 // Fragments of m8n8k4 (PTX ISA): A 8 x 4 row-major, lane holds A[lane / 4][lane % 4];
 // B 4 x 8 column-major, lane holds B[lane % 4][lane / 4]; C 8 x 8, lane holds
 // C[lane / 4][2 (lane % 4) + {0, 1}].

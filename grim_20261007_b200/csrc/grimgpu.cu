@@ -1946,11 +1946,12 @@ extern "C" int grim_zgesv_mixed(grim_handle_t h, int n, int nrhs, const void *A,
         // (no room for the copy: B waits for getrs)
         void *pB0 = nullptr;
         const size_t row = n * sizeof(double2);
-        const bool kept = grim_workspace(h, "gd_B0", row * nrhs, &pB0) == GRIM_OK;
+        const bool pivots = h->pivot_mode == GRIM_PIVOT_PARTIAL || h->pivot_mode == GRIM_PIVOT_TOURNAMENT;
+        const bool kept = pivots && grim_workspace(h, "gd_B0", row * nrhs, &pB0) == GRIM_OK;
         if (kept)
             GRIM_CHECK_CUDA(cudaMemcpy2DAsync(pB0, row, B, ldb * sizeof(double2), row, nrhs, cudaMemcpyDeviceToDevice,
                                               h->stream));
-        else
+        else if (pivots)
             cudaGetLastError();
         RhsForward fwd{(double2 *)B, ldb, nrhs};
         StreamTimer tf(h->stream);
