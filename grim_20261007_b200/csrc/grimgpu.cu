@@ -1837,6 +1837,15 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
     GRIM_CHECK_LAUNCH(h, "k_convert");
     double prev = INFINITY;
     int steps = 0;
+    auto correct = [&]() -> int {  // X += solve32(R)
+        k_convert<float2, double2><<<eg, 256, 0, h->stream>>>(n, nrhs, R, n, R32, n);
+        GRIM_CHECK_LAUNCH(h, "k_convert");
+        GRIM_TRY(solve32(R32));
+        k_add_update<float2><<<eg, 256, 0, h->stream>>>(n, nrhs, X, n, R32, n);
+        GRIM_CHECK_LAUNCH(h, "k_add_update");
+        ++steps;
+        return GRIM_OK;
+    };
     double berr = INFINITY, relres = INFINITY, first = -1.0;
     int status = GRIM_OK;
     // residuals on the integer tensor cores when the slice accumulators fit
@@ -1858,12 +1867,7 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
         }
         if (speculate && it == 0) {
             GRIM_CHECK_CUDA(cudaMemcpyAsync(sc + 4, sc + 1, 2 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-            k_convert<float2, double2><<<eg, 256, 0, h->stream>>>(n, nrhs, R, n, R32, n);
-            GRIM_CHECK_LAUNCH(h, "k_convert");
-            GRIM_TRY(solve32(R32));
-            k_add_update<float2><<<eg, 256, 0, h->stream>>>(n, nrhs, X, n, R32, n);
-            GRIM_CHECK_LAUNCH(h, "k_add_update");
-            ++steps;
+            GRIM_TRY(correct());
             continue;
         }
         double hv[4];
@@ -1884,7 +1888,20 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
         }
         if (first < 0) first = berr;
         const double measure = berr_test ? berr : relres;
-        if (std::isfinite(measure) && measure <= tol) break;
+        if (std::isfinite(measure) && measure <= tol) {
+            // An iterate that only just meets a backward-error target still carries the error of
+            // the last complex64 correction, which depends on how the factor happened to round:
+            // superellipses of N = 4099 (TE, 181 angles) came out up to 2.9e-9 off their FP64
+            // amplitudes, 34 times the backward error, and two builds that differ by rounding
+            // 3e-9 apart.  In the target's last decade the correction of the residual in hand
+            // goes in too (each takes off a factor of 20 or more there): below it the amplitudes
+            // are within 5e-10, what the integer slices of the residual leave.
+            if (berr_test && measure > 0.1 * tol && steps < max_iter) {
+                GRIM_TRY(correct());
+                GRIM_TRY(tc_err_check(h, "mixed-precision solve"));
+            }
+            break;
+        }
         if (!std::isfinite(measure) || measure >= prev * 0.98) {
             status = grim_fail(GRIM_ERR_NOT_CONVERGED, "mixed-precision refinement stalled; double LU required");
             break;
@@ -1894,12 +1911,7 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
             break;
         }
         prev = measure;
-        k_convert<float2, double2><<<eg, 256, 0, h->stream>>>(n, nrhs, R, n, R32, n);
-        GRIM_CHECK_LAUNCH(h, "k_convert");
-        GRIM_TRY(solve32(R32));
-        k_add_update<float2><<<eg, 256, 0, h->stream>>>(n, nrhs, X, n, R32, n);
-        GRIM_CHECK_LAUNCH(h, "k_add_update");
-        ++steps;
+        GRIM_TRY(correct());
     }
     GRIM_CHECK_CUDA(cudaMemcpy2DAsync(Bio, ldb * sizeof(double2), X, n * sizeof(double2), n * sizeof(double2), nrhs,
                                       cudaMemcpyDeviceToDevice, h->stream));
