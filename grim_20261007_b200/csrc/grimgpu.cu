@@ -1261,12 +1261,21 @@ static int rhs_interchanges(grim_context *h, int n, int nrhs, C *B, int64_t ldb,
     return GRIM_OK;
 }
 
-// Strip solves (k_trsolve_strip): a strip's time grows with n^2 on its one SM, the blocked
-// solve's with n (launches of 64-row blocks) until its GEMMs fill the chip.  One column meets
-// it at n = 2048 (1.87 ms either way), 181 columns at n = 3000 (4.0 ms); from 64 strips on the
-// strips fill the chip themselves (n = 4096, 720 columns 7.2 against 9.5 ms).
-static bool trsolve_wanted(int n, int nrhs) {
-    return tc_enabled() && (n <= 2048 || (n <= 3000 && nrhs >= 181) || nrhs >= 512);
+// Strip solves (k_trsolve_strip) or the blocked ones, both triangles in microseconds:
+//   strips   27 + waves (c n^2 + 9 blocks), waves of sm_count strips of eight columns, 64-row
+//            blocks; c = 3.3e-4, or 4.0e-4 where every column starts on a 128-byte line (the four
+//            columns that a warp reads at a time then meet in the caches: N = 2048 with leading
+//            dimension 2048 1.98 ms, 2050 1.68);
+//   blocked  10 + 38 blocks (four launches each) + 5.0e-7 n^2 nrhs (the GEMMs).
+// The cheaper of the two is at most 9 % slower than the faster one over n = 48 .. 12000 and 1 ..
+// 3600 columns, 0.3 % on average.  Strips against blocked: n = 333, 37 columns 0.135 / 0.256 ms;
+// n = 2048, 16 columns 1.98 / 1.32, 361 1.98 / 2.04, 720 1.98 / 2.60; n = 4096, 512 7.17 / 6.60, 720
+// 7.17 / 7.88; n = 8192, 512 27.3 / 20.6, 1024 27.4 / 42.6; n = 64, 2400 (three waves) 0.062 / 0.053.
+static bool trsolve_wanted(const grim_context *h, int n, int64_t lda, int nrhs) {
+    const double n2 = (double)n * n, blocks = ceil_div(n, NB);
+    const int waves = ceil_div(ceil_div(nrhs, TRS_COLS), h->sm_count);
+    return tc_enabled() && 27.0 + waves * ((lda % 8 ? 3.3e-4 : 4.0e-4) * n2 + 9.0 * blocks) <=
+                               10.0 + 38.0 * blocks + 5.0e-7 * n2 * nrhs;
 }
 
 template <bool UPPER>
@@ -1288,7 +1297,7 @@ static int getrs_upper(grim_context *h, int n, int nrhs, const C *LU, int64_t ld
     const int npan = ceil_div(n, NB);
     const size_t tri = (size_t)(NB * NBP + NB) * sizeof(C);
     if constexpr (sizeof(C) == sizeof(double2)) {
-        if (trsolve_wanted(n, nrhs)) return trsolve_strip<true>(h, n, nrhs, LU, lda, B, ldb);
+        if (trsolve_wanted(h, n, lda, nrhs)) return trsolve_strip<true>(h, n, nrhs, LU, lda, B, ldb);
     }
     const int ctiles = ceil_div(nrhs, TRSM_COLS);
     for (int p = npan - 1; p >= 0; --p) {
@@ -1308,7 +1317,7 @@ static int getrs_apply(grim_context *h, int n, int nrhs, const C *LU, int64_t ld
     const size_t tri = (size_t)(NB * NBP + NB) * sizeof(C);
     GRIM_TRY(rhs_interchanges<C>(h, n, nrhs, B, ldb, ipiv, ident));
     if constexpr (sizeof(C) == sizeof(double2)) {
-        if (trsolve_wanted(n, nrhs)) {
+        if (trsolve_wanted(h, n, lda, nrhs)) {
             GRIM_TRY((trsolve_strip<false>(h, n, nrhs, LU, lda, B, ldb)));
             return getrs_upper<C>(h, n, nrhs, LU, lda, B, ldb);
         }

@@ -93,6 +93,31 @@ def test_elimination_beside_the_factorization(n, nrhs, mode):
     assert np.max(res / den) < 1e-14
 
 
+# one, two and four panels a launch of the forward elimination (a launch is due by its rows from
+# 1536 on, else by four panels); backward substitutions in strips and blocked on both sides of
+# the rule (few columns above 1500 rows and third waves of strips take the blocked one)
+@pytest.mark.parametrize('n, nrhs', [(64, 2369), (65, 1184), (65, 1185), (513, 3553), (1400, 9), (1601, 9), (1601, 361),
+                                     (2048, 33), (2113, 9), (2113, 361), (3073, 8), (3073, 720)])
+@pytest.mark.parametrize('pivot', ['partial', None])
+def test_large_solves_on_both_sides_of_the_strip_rule(n, nrhs, pivot):
+    """Whole solves (elimination beside a partial-pivoting factorization, or getrs after a
+    certified one): normwise backward error of every column."""
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.device import context, ptr
+    ctx = context()
+    gen = torch.Generator(device='cuda').manual_seed(n + nrhs)
+    at = torch.randn((n, n), dtype=torch.complex128, device='cuda', generator=gen)
+    bt = torch.randn((nrhs, n), dtype=torch.complex128, device='cuda', generator=gen)
+    x, info = bt.clone(), ctypes.c_int(-1)
+    mode = _lib.PREC_FP64 | (_lib.PREC_PARTIAL_PIVOT if pivot else 0)
+    _lib.check(ctx.lib.grim_zgesv_mixed(ctx.h, n, nrhs, ptr(at), n, None, 0, ptr(x), n, mode, 1e-10, 0,
+                                        ctypes.byref(info), None))
+    assert info.value == 0
+    res = (x @ at - bt).abs().amax(1)  # rows of the tensors are columns of the matrices
+    den = at.abs().sum(0).max() * x.abs().amax(1) + bt.abs().amax(1)
+    assert float((res / den).max()) < 1e-14
+
+
 def test_singular_matrix_leaves_the_right_hand_sides():
     from grim_20261007_b200 import _lib
     n = 300
