@@ -2837,6 +2837,14 @@ extern "C" int grim_far_block_fresh(int64_t mb, int64_t nb, int q, int width, co
                           mirrored, k_re, k_im, intervals, bounds, degree, coeff, acc_s, acc_k, acc_kt);
 }
 
+// dst (rows x cols, column-major, contiguous) = src (row-major, contiguous).
+static int transpose(grim_context *h, int rows, int cols, const void *src, void *dst) {
+    const dim3 grid(ceil_div(cols, 32), std::min(ceil_div(rows, 32), 65535));
+    k_transpose<<<grid, dim3(32, 8), 0, h->stream>>>(rows, cols, (const double2 *)src, cols, (double2 *)dst, rows);
+    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    return GRIM_OK;
+}
+
 // B1 drop-in with host buffers.
 extern "C" int grim_zgesv_batched(grim_handle_t h, int n, int nrhs, const double *A, int lda, double *B, int ldb,
                                   int precision_mode, int *info) {
@@ -2879,15 +2887,10 @@ extern "C" int grim_zgesv_rowmajor(grim_handle_t h, int n, int nrhs, const doubl
     double2 *ra = (double2 *)pr, *rb = ra + an;
     GRIM_TRY(stage_copy(h, {{ra, const_cast<double *>(A), an * sizeof(double2)},
                             {rb, const_cast<double *>(B), bn * sizeof(double2)}}, true));
-    const dim3 block(32, 8);
-    k_transpose<<<dim3(ceil_div(n, 32), ceil_div(n, 32)), block, 0, h->stream>>>(n, n, ra, n, (double2 *)pa, n);
-    GRIM_CHECK_LAUNCH(h, "k_transpose");
-    k_transpose<<<dim3(ceil_div(nrhs, 32), ceil_div(n, 32)), block, 0, h->stream>>>(n, nrhs, rb, nrhs, (double2 *)pb, n);
-    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    GRIM_TRY(transpose(h, n, n, ra, pa));
+    GRIM_TRY(transpose(h, n, nrhs, rb, pb));
     GRIM_TRY(grim_zgesv_mixed(h, n, nrhs, pa, n, nullptr, 0, pb, n, precision_mode, 2e-12, 10, info, nullptr));
-    k_transpose<<<dim3(ceil_div(n, 32), ceil_div(nrhs, 32)), block, 0, h->stream>>>(nrhs, n, (const double2 *)pb, n, rb,
-                                                                                    nrhs);
-    GRIM_CHECK_LAUNCH(h, "k_transpose");
+    GRIM_TRY(transpose(h, nrhs, n, pb, rb));
     return stage_copy(h, {{rb, X, bn * sizeof(double2)}}, false);
 }
 

@@ -121,16 +121,19 @@ static int stage_copy(grim_context *h, const std::vector<HostCopy> &list, bool u
     return GRIM_OK;
 }
 
-// dst[c][r] = src[r][c] (rows x cols, row-major, to column-major leading dimension ldd).
+// dst[c][r] = src[r][c] (rows x cols, row-major, to column-major leading dimension ldd); the grid
+// covers the columns, its y extent steps over the rows.
 __global__ void k_transpose(int rows, int cols, const double2 *__restrict__ src, int64_t lds, double2 *__restrict__ dst,
                             int64_t ldd) {
     __shared__ double2 tile[32][33];
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y)
-        if (r0 + i < rows && c0 + threadIdx.x < cols)
-            tile[i][threadIdx.x] = src[(int64_t)(r0 + i) * lds + c0 + threadIdx.x];
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y)
-        if (c0 + i < cols && r0 + threadIdx.x < rows)
-            dst[(int64_t)(c0 + i) * ldd + r0 + threadIdx.x] = tile[threadIdx.x][i];
+    const int c0 = blockIdx.x * 32;
+    for (int64_t r0 = (int64_t)blockIdx.y * 32; r0 < rows; r0 += (int64_t)gridDim.y * 32) {
+        for (int i = threadIdx.y; i < 32; i += blockDim.y)
+            if (r0 + i < rows && c0 + threadIdx.x < cols) tile[i][threadIdx.x] = src[(r0 + i) * lds + c0 + threadIdx.x];
+        __syncthreads();
+        for (int i = threadIdx.y; i < 32; i += blockDim.y)
+            if (c0 + i < cols && r0 + threadIdx.x < rows)
+                dst[(int64_t)(c0 + i) * ldd + r0 + threadIdx.x] = tile[threadIdx.x][i];
+        __syncthreads();
+    }
 }

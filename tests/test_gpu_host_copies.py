@@ -33,6 +33,20 @@ def test_dense_hook_takes_every_layout(n, nrhs, layout):
     assert v.shape == (n,) and np.max(np.abs(v - x[:, 0])) <= 1e-13 * np.max(np.abs(x))
 
 
+def test_row_major_systems_take_millions_of_columns():
+    """More 32-column tiles of the solution than a grid's y extent."""
+    import ctypes
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.device import context
+    ctx = context()
+    a = np.array([[2.0 + 1.0j, 0.5], [1.0j, 3.0]])
+    b = np.stack([np.arange(2_100_000) + 0j, np.arange(2_100_000)[::-1] * 1j])
+    x, info = np.empty_like(b), ctypes.c_int(-1)
+    _lib.check(ctx.lib.grim_zgesv_rowmajor(ctx.h, 2, b.shape[1], a.ctypes.data, b.ctypes.data, x.ctypes.data,
+                                           _lib.PREC_FP64, ctypes.byref(info)))
+    assert np.max(np.abs(a @ x - b)) <= 1e-14 * np.max(np.abs(b))
+
+
 @pytest.mark.parametrize('rows, cols', [(3, 2), (130, 131), (181, 182), (300, 257)])
 def test_far_block_from_zero_equals_accumulating(rows, cols):
     """Fresh accumulators equal sums into zeros; sums into other values keep them."""
