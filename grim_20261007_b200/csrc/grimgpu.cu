@@ -149,6 +149,14 @@ int grim_workspace(grim_context *h, const char *name, size_t bytes, void **out) 
     return GRIM_OK;
 }
 
+// Gives a named workspace back (after the work queued on the handle's stream).
+static void grim_drop_workspace(grim_context *h, const char *name) {
+    auto it = h->ws.find(name);
+    if (it == h->ws.end()) return;
+    cudaFreeAsync(it->second.first, h->stream);
+    h->ws.erase(it);
+}
+
 // ============================================================== context API
 extern "C" int grim_version(void) { return 1; }
 extern "C" const char *grim_last_error(void) { return g_last_error.c_str(); }
@@ -1626,6 +1634,9 @@ static int oz_bn(int S, int nrhs, int Rp, int sms) {
 // int32 accumulators hold S products of 2n terms of at most 64^2.
 static bool oz_fits(int n, int S) { return (double)S * 2.0 * n * 64.0 * 64.0 < 2147483647.0; }
 
+// Residuals on the integer tensor cores pay from these sizes on.
+static bool oz_wanted(int n, int nrhs, int S) { return tc_enabled() && n >= 256 && nrhs >= 16 && oz_fits(n, S); }
+
 template <typename TA>
 static int oz_prepare_a(grim_context *h, int n, const TA *A, int64_t lda, int S, OzA *out) {
     if (!oz_supported(S)) return grim_fail(GRIM_ERR_ARGUMENT, "integer-slice residual: unsupported slice count");
@@ -1860,7 +1871,7 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
     // residuals on the integer tensor cores when the slice accumulators fit
     OzA qa;
     const int oz_s = oz_slices_for(berr_test, tol);
-    const bool use_oz = tc_enabled() && n >= 256 && nrhs >= 16 && oz_fits(n, oz_s);
+    const bool use_oz = oz_wanted(n, nrhs, oz_s);
     if (use_oz) GRIM_TRY(oz_prepare_a(h, n, Ares, ldres, oz_s, &qa));
     // A backward-error target below complex64 accuracy always needs a correction: the first
     // one is then queued without reading the initial residual's norms on the host (they
@@ -2873,25 +2884,43 @@ extern "C" int grim_zgesv_batched(grim_handle_t h, int n, int nrhs, const double
 }
 
 // The same for row-major (C-order) A (n x n), B and X (n x nrhs), B kept: the transposes that
-// a column-major call costs the host (3 ms at n = 900) run on the device.
+// a column-major call costs the host (3 ms at n = 900) run on the device.  The rows land in the
+// buffer that the solve itself needs and has not filled yet (the factor, or the residual's
+// slices of A), one matrix after the other when both do not fit there with 64 MiB to spare, so
+// that the call needs and keeps no more device memory than a column-major one.
+#define ROWS_EXTRA ((size_t)64 << 20)
 extern "C" int grim_zgesv_rowmajor(grim_handle_t h, int n, int nrhs, const double *A, const double *B, double *X,
                                    int precision_mode, int *info) {
     if (!h || n <= 0 || nrhs <= 0 || !A || !B || !X)
         return grim_fail(GRIM_ERR_ARGUMENT, "grim_zgesv_rowmajor: bad arguments");
     DeviceGuard g(h->device);
-    const size_t an = (size_t)n * n, bn = (size_t)n * nrhs;
+    const size_t an = (size_t)n * n * sizeof(double2), bn = (size_t)n * nrhs * sizeof(double2);
+    const int prec = precision_mode & ~(GRIM_PREC_STATIC_PIVOT | GRIM_PREC_PARTIAL_PIVOT | GRIM_PREC_TOURNAMENT_PIVOT);
+    const bool own = prec != GRIM_PREC_FP64 && !oz_wanted(n, nrhs, 8);  // neither buffer is used: one for the call
+    const char *name = own ? "h_rows" : prec == GRIM_PREC_FP64 ? "sv_lu64" : "oz_q";
+    const bool both = an + bn <= ROWS_EXTRA;
     void *pr = nullptr, *pa = nullptr, *pb = nullptr;
-    GRIM_TRY(grim_workspace(h, "h_rows", (an + bn) * sizeof(double2), &pr));
-    GRIM_TRY(grim_workspace(h, "h_A", an * sizeof(double2), &pa));
-    GRIM_TRY(grim_workspace(h, "h_B", bn * sizeof(double2), &pb));
-    double2 *ra = (double2 *)pr, *rb = ra + an;
-    GRIM_TRY(stage_copy(h, {{ra, const_cast<double *>(A), an * sizeof(double2)},
-                            {rb, const_cast<double *>(B), bn * sizeof(double2)}}, true));
-    GRIM_TRY(transpose(h, n, n, ra, pa));
-    GRIM_TRY(transpose(h, n, nrhs, rb, pb));
+    GRIM_TRY(grim_workspace(h, name, both ? an + bn : std::max(an, bn), &pr));
+    GRIM_TRY(grim_workspace(h, "h_A", an, &pa));
+    GRIM_TRY(grim_workspace(h, "h_B", bn, &pb));
+    const HostCopy ca{pr, const_cast<double *>(A), an}, cb{both ? (char *)pr + an : pr, const_cast<double *>(B), bn};
+    if (both) {
+        GRIM_TRY(stage_copy(h, {ca, cb}, true));
+        GRIM_TRY(transpose(h, n, n, ca.device, pa));
+    } else {
+        GRIM_TRY(stage_copy(h, {ca}, true));
+        GRIM_TRY(transpose(h, n, n, ca.device, pa));
+        GRIM_TRY(stage_copy(h, {cb}, true));
+    }
+    GRIM_TRY(transpose(h, n, nrhs, cb.device, pb));
+    if (own && !both) grim_drop_workspace(h, name);
     GRIM_TRY(grim_zgesv_mixed(h, n, nrhs, pa, n, nullptr, 0, pb, n, precision_mode, 2e-12, 10, info, nullptr));
-    GRIM_TRY(transpose(h, nrhs, n, pb, rb));
-    return stage_copy(h, {{rb, X, bn * sizeof(double2)}}, false);
+    // the factor and the slices are done with
+    GRIM_TRY(grim_workspace(h, name, bn, &pr));
+    GRIM_TRY(transpose(h, nrhs, n, pb, pr));
+    GRIM_TRY(stage_copy(h, {{pr, X, bn}}, false));
+    if (own && !both) grim_drop_workspace(h, name);
+    return GRIM_OK;
 }
 
 // ============================================================== profiling

@@ -33,6 +33,43 @@ def test_dense_hook_takes_every_layout(n, nrhs, layout):
     assert v.shape == (n,) and np.max(np.abs(v - x[:, 0])) <= 1e-13 * np.max(np.abs(x))
 
 
+@pytest.mark.parametrize('mode, nrhs', [('PREC_FP64', 64), ('PREC_FP64', 3500), ('PREC_MIXED', 64), ('PREC_MIXED', 3)])
+def test_row_major_systems_keep_no_more_memory_than_column_major_ones(mode, nrhs):
+    """The device memory that a call leaves held, and the answer with its rows in a buffer of the
+    solve (a matrix of 140 MB: one host array after the other goes through it)."""
+    import ctypes
+    from grim_20261007_b200 import _lib
+    lib = _lib.load()
+    n = 3000
+    rng = np.random.default_rng(nrhs)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * n ** 0.5 * np.eye(n)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    held, xs = [], []
+    for rows in (False, True):
+        h, info, free, total = ctypes.c_void_p(), ctypes.c_int(-1), ctypes.c_size_t(), ctypes.c_size_t()
+        _lib.check(lib.grim_create(0, ctypes.byref(h)))
+        try:
+            _lib.check(lib.grim_mem_info(h, ctypes.byref(free), ctypes.byref(total)))
+            before = free.value
+            if rows:
+                x = np.empty_like(b)
+                _lib.check(lib.grim_zgesv_rowmajor(h, n, nrhs, a.ctypes.data, b.ctypes.data, x.ctypes.data,
+                                                   getattr(_lib, mode), ctypes.byref(info)))
+            else:
+                af, x = np.asfortranarray(a), np.asfortranarray(b)
+                _lib.check(lib.grim_zgesv_batched(h, n, nrhs, af.ctypes.data, n, x.ctypes.data, n, getattr(_lib, mode),
+                                                  ctypes.byref(info)))
+            _lib.check(lib.grim_synchronize(h))
+            _lib.check(lib.grim_mem_info(h, ctypes.byref(free), ctypes.byref(total)))
+            held.append(before - free.value)
+            xs.append(x)
+        finally:
+            lib.grim_destroy(h)
+    assert np.max(np.abs(xs[1] - xs[0])) <= 1e-11 * np.max(np.abs(xs[0]))
+    extra = max(0, nrhs - n) * n * 16  # right-hand sides wider than the matrix
+    assert held[1] <= held[0] + extra + (64 << 20), held
+
+
 def test_row_major_systems_take_millions_of_columns():
     """More 32-column tiles of the solution than a grid's y extent."""
     import ctypes
