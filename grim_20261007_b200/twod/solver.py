@@ -133,9 +133,11 @@ def _solve_dense_gpu(a_eval, rhs_eval):
     info = _lib.ctypes.c_int(0)
     mode = _lib.PREC_MIXED if requested_precision() == 'mixed' else _lib.PREC_FP64
     # a C-order matrix (with right-hand sides in either order) goes up as it is and is transposed
-    # on the device, three launches that a small one does not repay (n = 64 0.32 against 0.30 ms,
-    # n = 100 0.43 against 0.53); any other layout is laid out column-major here
-    rows = n >= 80 and a.flags.c_contiguous and not a.flags.f_contiguous
+    # on the device, three launches that small systems do not repay (100 x 1 0.315 against 0.298
+    # ms, 64 x 60 0.206 against 0.213, 16 x 400 0.180 against 0.192, 60 x 3000 0.84 against 2.59:
+    # the right-hand sides are laid out three times on the host, the matrix once); any other
+    # layout is laid out column-major here
+    rows = n * (n + 3 * nrhs) >= 15000 and a.flags.c_contiguous and not a.flags.f_contiguous
     if rows:
         b_in = np.ascontiguousarray(b2)
         x = np.empty((n, nrhs), dtype=np.complex128)

@@ -33,6 +33,17 @@ def test_dense_hook_takes_every_layout(n, nrhs, layout):
     assert v.shape == (n,) and np.max(np.abs(v - x[:, 0])) <= 1e-13 * np.max(np.abs(x))
 
 
+@pytest.mark.parametrize('n, nrhs', [(2, 2600), (16, 300), (16, 310), (60, 70), (60, 2500), (121, 1), (122, 1)])
+def test_dense_hook_on_both_sides_of_the_row_major_rule(n, nrhs):
+    """n (n + 3 nrhs) from 15000 on goes up row-major; few rows and many columns among them."""
+    from grim_20261007_b200.twod.solver import _solve_dense_gpu
+    rng = np.random.default_rng(n + nrhs)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * n ** 0.5 * np.eye(n)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    x, _name = _solve_dense_gpu(a, b)
+    assert np.max(np.abs(a @ x - b)) < 1e-14 * (np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x)))
+
+
 @pytest.mark.parametrize('mode, nrhs', [('PREC_FP64', 64), ('PREC_FP64', 3500), ('PREC_MIXED', 64), ('PREC_MIXED', 3)])
 def test_row_major_systems_keep_no_more_memory_than_column_major_ones(mode, nrhs):
     """The device memory that a call leaves held, and the answer with its rows in a buffer of the
