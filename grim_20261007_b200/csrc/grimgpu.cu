@@ -547,6 +547,7 @@ template <bool NEG, bool BETA>
 static int dmma_gemm(grim_context *h, int M, int N, int K, const double2 *A, int64_t lda, const double2 *B,
                      int64_t ldb, double2 *C, int64_t ldc) {
     auto load = [&](int bm, int bn, double loss) {
+        if (ceil_div(N, bn) > 65535) return (double)INFINITY;  // the grid's y extent
         const int64_t tiles = (int64_t)ceil_div(M, bm) * ceil_div(N, bn);
         return (double)((tiles + h->sm_count - 1) / h->sm_count) * bm * bn * loss;
     };

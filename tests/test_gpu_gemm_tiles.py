@@ -31,3 +31,17 @@ def test_residual_equals_numpy(n, nrhs):
     # rounding of an n-term complex dot product
     bound = 8.0 * np.finfo(float).eps * n ** 0.5 * (np.max(np.abs(b)) + n ** 0.5 * np.max(np.abs(a)) * np.max(np.abs(x)))
     assert np.max(np.abs(out[:, :n].T - (b - a @ x))) <= bound
+
+
+def test_millions_of_columns_keep_to_the_wide_tiles():
+    """32 columns a tile would need more tiles than a grid's y extent."""
+    from grim_20261007_b200 import _lib
+    from grim_20261007_b200.device import context, ptr
+    ctx = context()
+    n, nrhs = 16, 2_100_000
+    gen = torch.Generator(device='cuda').manual_seed(1)
+    a, x, b = (torch.randn((c, n), dtype=torch.complex128, device='cuda', generator=gen) for c in (n, nrhs, nrhs))
+    r = torch.empty_like(b)
+    _lib.check(ctx.lib.grim_residual(ctx.h, n, nrhs, ptr(a), n, 0, ptr(x), n, ptr(b), n, ptr(r), n, 0))
+    ref = b - x @ a  # rows of the tensors are columns of the matrices
+    assert float((r - ref).abs().max()) <= 8.0 * np.finfo(float).eps * 4.0 * n * float(x.abs().max() * a.abs().max())
