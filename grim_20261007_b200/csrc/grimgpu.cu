@@ -761,13 +761,11 @@ static const char *kname(const char *base, size_t csize) {
 
 // Streams and events of the look-ahead (created once per handle).
 static int lookahead_streams(grim_context *h, int nevents) {
-    if (!h->chain) {
-        int least = 0, greatest = 0;
-        GRIM_CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->chain, cudaStreamNonBlocking, greatest));
-        GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->bulk, cudaStreamNonBlocking, least));
-        GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->forward, cudaStreamNonBlocking, least));
-    }
+    int least = 0, greatest = 0;
+    if (!h->forward) GRIM_CHECK_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    if (!h->chain) GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->chain, cudaStreamNonBlocking, greatest));
+    if (!h->bulk) GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->bulk, cudaStreamNonBlocking, least));
+    if (!h->forward) GRIM_CHECK_CUDA(cudaStreamCreateWithPriority(&h->forward, cudaStreamNonBlocking, least));
     while ((int)h->events.size() < nevents) {
         cudaEvent_t e;
         GRIM_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1039,6 +1037,15 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
     int *flags = (int *)p_flags;
     int *d_info = flags, *d_pivoted = flags + 1, *cert = flags + 2, *swapped = cert + npan, *counter = swapped + npan;
     GRIM_CHECK_CUDA(cudaMemsetAsync(flags, 0, (size_t)(2 + 3 * npan) * sizeof(int), h->stream));
+    int *moves_all = nullptr;  // pivoted panels: the row moves of each (GEPP_MOVES_STRIDE)
+    const bool tournament = h->pivot_mode == GRIM_PIVOT_TOURNAMENT;
+    TsluWs tws;
+    if (h->pivot_mode == GRIM_PIVOT_PARTIAL || tournament) {
+        void *pm = nullptr;
+        GRIM_TRY(grim_workspace(h, "lu_moves_all", (size_t)npan * GEPP_MOVES_STRIDE * sizeof(int), &pm));
+        moves_all = (int *)pm;
+        if (tournament) GRIM_TRY(tslu_workspace<C>(h, n, &tws));
+    }
     const size_t tri = (size_t)(NB * NBP + NB) * sizeof(C);
     const bool split = !h->profiling;
     const cudaStream_t caller = h->stream;
@@ -1059,15 +1066,6 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
     }
     int status = GRIM_OK;
     bool wide_pending = false;
-    int *moves_all = nullptr;  // pivoted panels: the row moves of each (GEPP_MOVES_STRIDE)
-    const bool tournament = h->pivot_mode == GRIM_PIVOT_TOURNAMENT;
-    TsluWs tws;
-    if (h->pivot_mode == GRIM_PIVOT_PARTIAL || tournament) {
-        void *pm = nullptr;
-        GRIM_TRY(grim_workspace(h, "lu_moves_all", (size_t)npan * GEPP_MOVES_STRIDE * sizeof(int), &pm));
-        moves_all = (int *)pm;
-        if (tournament) GRIM_TRY(tslu_workspace<C>(h, n, &tws));
-    }
     int fwd_next = 0, fwd_rows = 0;
     for (int p = 0; p < npan && status == GRIM_OK && moves_all; ++p) {
         // partial pivoting: the panel on a cluster, then the trailing columns' row moves and
@@ -1110,7 +1108,9 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
             fwd_rows += rest;
         }
         if (wide_pending) {
-            GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0));
+            status = grim_cuda_status(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0),
+                                      "cudaStreamWaitEvent");
+            if (status != GRIM_OK) break;
             wide_pending = false;
         }
         if (rest > 0) {
@@ -1134,7 +1134,9 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
         status = grim_launch_status(h, kname("k_diag_lu", sizeof(C)), 8.0 * nbj * nbj * nbj / 3.0, 0);
         if (status != GRIM_OK) break;
         if (wide_pending) {
-            GRIM_CHECK_CUDA(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0));
+            status = grim_cuda_status(cudaStreamWaitEvent(h->stream, h->events[2 + npan + p - 1], 0),
+                                      "cudaStreamWaitEvent");
+            if (status != GRIM_OK) break;
             wide_pending = false;
         }
         const int rest = n - j - nbj;
