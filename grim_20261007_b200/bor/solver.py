@@ -113,10 +113,17 @@ MIRROR_ASYMMETRY_MAX = 1e-12
 BOR_LINEAR_BACKWARD_ERROR_MAX = 1.0e-12
 BOR_LINEAR_RESIDUAL_MAX = 1.0e-8
 GATE_REFINEMENT_STEPS = 2
-# the gate's residual: the FP64 GEMM, or for the largest mode systems int8 slices on the integer
-# tensor cores at its accuracy (n = 800, 722 columns 0.17 against 0.28 ms; n = 2048, 720 0.97
-# against 0.88 ms)
-GATE_SLICES, GATE_SLICES_MIN_ORDER = 8, 2048
+GATE_SLICES = 8
+
+
+def gate_slices(n, nrhs):
+    """Slices of the gate's residual: 0 for the FP64 GEMM, GATE_SLICES for int8 slices on the
+    integer tensor cores at its accuracy.  The slices cost a pass over the matrix that few
+    columns do not repay and half the GEMM's time a column, in steps of partly filled waves
+    either way: n = 800, 722 columns 0.17 ms FP64 against 0.28; n = 1402, 182 0.65 of the slices'
+    time, 1200 1.65; n = 2400, 182 1.0, 1200 1.55; n = 4002, 74 0.5, 362 1.37.  Over n = 600 .. 4002
+    and 2 .. 3000 columns the choice is 2.5 % off the faster one on average, 28 % at most."""
+    return GATE_SLICES if nrhs >= 300 + 5e8 / (float(n) * n) else 0
 
 
 def solution_errors(Z, X, B, R, maxes, ctx=None, berr=None, relres=None):
@@ -128,9 +135,9 @@ def solution_errors(Z, X, B, R, maxes, ctx=None, berr=None, relres=None):
     before reading the results."""
     ctx = ctx or context()
     n, nrhs = int(B.shape[1]), int(B.shape[0])
-    slices = GATE_SLICES if n >= GATE_SLICES_MIN_ORDER else 0
-    _lib.check(ctx.lib.grim_solution_errors(ctx.h, n, nrhs, ptr(Z), n, ptr(X), n, ptr(B), n, ptr(R), n, slices,
-                                            ptr(berr), ptr(relres), ptr(maxes)), 'grim_solution_errors')
+    _lib.check(ctx.lib.grim_solution_errors(ctx.h, n, nrhs, ptr(Z), n, ptr(X), n, ptr(B), n, ptr(R), n,
+                                            gate_slices(n, nrhs), ptr(berr), ptr(relres), ptr(maxes)),
+               'grim_solution_errors')
 
 
 def release_limit(prec, tol):

@@ -191,3 +191,10 @@ def test_finish_modes_decisions_without_a_device(monkeypatch):
     with pytest.raises(RuntimeError, match='m=1 estimated 1-norm condition'):
         B._finish_modes(None, [0, 1], None, bad, 1e-10, Ctx(), True)
     assert redone == []
+
+
+@pytest.mark.parametrize('n, nrhs, slices', [(800, 722, 0), (100, 1440, 0), (1402, 182, 0), (1402, 1200, 8),
+                                             (2400, 74, 0), (2400, 1200, 8), (4002, 2, 0), (4002, 400, 8)])
+def test_gate_residual_takes_the_slices_where_they_are_faster(n, nrhs, slices):
+    """Both unknowns count: sizes on either side, all of them more than a quarter apart in time."""
+    assert B.gate_slices(n, nrhs) == slices
