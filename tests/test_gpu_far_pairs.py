@@ -97,3 +97,39 @@ def test_converged_orders_hold_every_floor(kl, floor, pol, monkeypatch):
     eps = np.finfo(float).eps
     order_error = 2e-11 if pol == 'TM' else 0.0  # 5- to 8-point rules of the TM table
     assert np.all(np.abs(z[rows, cols] - ref) <= (8.0 * eps * (8.0 + k * dist) + order_error) * scale)
+
+
+@pytest.mark.parametrize('stretch', [0.0, 0.5])
+@pytest.mark.parametrize('kl', [0.02, 0.3, 0.8, 1.6, 2.6, 3.6])
+@pytest.mark.parametrize('floor', [8, 16])
+def test_converged_orders_hold_beside_the_near_pairs(kl, floor, stretch, monkeypatch):
+    """TE entries of element pairs three to nine lengths apart (orders 10, 9, 8 and, past |k| L = 3,
+    16), lengths of up to 1 : 2 and 1 : 5, against a 24-point rule."""
+    from grim_20261007_b200.device import to_host_matrix
+    from grim_20261007_b200.twod.galerkin import GalerkinBody
+    monkeypatch.setattr(GalerkinBody, 'far_min_order', lambda self, k, p: floor)
+    n = 400
+    theta = -2.0 * np.pi * (np.arange(n) + np.random.default_rng(2).uniform(-0.15, 0.15, n)) / n
+    theta = theta + stretch * np.sin(theta)
+    drawn = np.stack([np.cos(theta), 0.8 * np.sin(theta)], axis=1)
+    a = drawn[(-np.arange(n)) % n]
+    b = np.roll(a, -1, axis=0)
+    length, mid = np.hypot(*(b - a).T), 0.5 * (a + b)
+    k = kl / length.max()
+    z = to_host_matrix(GalerkinBody([drawn]).fill_matrix(k, 'TE'))
+    rows = np.arange(n).repeat(6)
+    cols = (rows + np.tile([4, 5, 6, 7, 8, 9], n)) % n
+    ratio = np.min([np.hypot(*(mid[(rows - p) % n] - mid[(cols - q) % n]).T) /
+                    np.maximum(length[(rows - p) % n], length[(cols - q) % n]) for p in (0, 1) for q in (0, 1)], axis=0)
+    sel = ratio > 3.001  # all four element pairs far
+    rows, cols = rows[sel], cols[sel]
+    assert np.min(ratio[sel]) < 3.2 and np.max(ratio[sel]) > 7.0
+    ref = _far_entries(drawn, k, 'TE', rows, cols, order=24)
+    # every kernel value a few ulp, its phase and its distance of coordinates of order 1
+    dist = np.hypot(*(a[rows] - a[cols]).T)
+    near = np.maximum(dist - 1.5 * length.max(), 0.5 * dist)
+    big = length.max()
+    g = 0.25 * np.hypot(special.j0(k * near), special.y0(k * near))
+    h = 0.25 * k * np.hypot(special.j1(k * near), special.y1(k * near))
+    scale = 4.0 * (h * big ** 2 + k * g * big ** 2 + g / k)
+    assert np.all(np.abs(z[rows, cols] - ref) <= 8.0 * np.finfo(float).eps * (8.0 + k * dist) * scale)

@@ -97,6 +97,24 @@ def test_partial_pivoting_cgetrf_large_is_a_partial_pivoting_lu(ctx):
     assert np.max(np.abs(pa - low @ up)) <= 1e-4 * np.max(np.abs(a))
 
 
+@pytest.mark.parametrize('n', [2049, 2100, 3500, 4096, 4097])
+def test_partial_pivoting_cgetrf_of_tall_panels_is_a_partial_pivoting_lu(ctx, n):
+    """complex64 panels of 2049 to 4096 rows (256 register-resident rows a CTA, the last CTA
+    ragged) and one that starts above them in shared memory: P A = L U and |l| <= sqrt 2 as at
+    n = 2048, the residual's bound grown with n."""
+    from grim_20261007_b200 import _lib
+    a = torch.complex(*torch.randn((2, n, n), device='cuda', generator=torch.Generator(device='cuda').manual_seed(n)))
+    t, ipiv, info = _getrf(ctx, a.T.cpu().numpy(), complex64=True, pivot=_lib.PIVOT_PARTIAL)
+    assert info == 0
+    lu = t.T.to(torch.complex128)  # rows of t are columns
+    low, up = torch.tril(lu, -1), torch.triu(lu)
+    assert float(low.abs().max()) <= np.sqrt(2.0) * (1.0 + 1e-5)
+    low += torch.eye(n, device='cuda')
+    perm = torch.from_numpy(_lapack_perm(ipiv.cpu().numpy())).cuda()
+    pa = a.T.to(torch.complex128)[perm]
+    assert float((pa - low @ up).abs().max()) <= 1e-4 * (n / 2048.0) * float(a.abs().max())
+
+
 @pytest.mark.parametrize('n', [160, 700])
 def test_partial_pivoting_cgetrf_matches_lapack(ctx, n):
     from grim_20261007_b200 import _lib
