@@ -1094,7 +1094,7 @@ static int getrf_impl(grim_context *h, int n, C *A, int64_t lda, int *ipiv, int 
             // of the last wide update) and is issued after it: a cluster of 16 CTAs finds no room
             // once strips hold half the SMs
             const bool last = rest == 0, due = fwd_rows >= TRS_FWD_ROWS || p - fwd_next >= TRS_FWD_PANELS;
-            if (forward && (last || (due && rest + nbj > NB))) {
+            if (forward && (last || due)) {
                 if (last) status = grim_cuda_status(cudaEventRecord(h->events[2 + p], h->stream), "cudaEventRecord");
                 if (status == GRIM_OK)
                     status = grim_cuda_status(

@@ -39,13 +39,7 @@ struct HankelTab {
         e[4][GH_DEG_E + 1];
 };
 __constant__ HankelTab c_hankel;
-static HankelTab h_hankel;  // the host's copy (upload, host checks)
-
-#ifdef __CUDA_ARCH__
-#define GH_TAB c_hankel
-#else
-#define GH_TAB h_hankel
-#endif
+static HankelTab h_hankel;  // computed here, uploaded to every device
 
 // ------------------------------------------------------------------ host: the coefficients
 static void hankel_pq(long double x, int nu, long double &P, long double &Q) {
@@ -140,20 +134,16 @@ static void hankel_tables() {
 }
 
 // ------------------------------------------------------------------ device
-__host__ __device__ __forceinline__ double gh_fourth_root_estimate(double u) {
-#ifdef __CUDA_ARCH__
+__device__ __forceinline__ double gh_fourth_root_estimate(double u) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"((float)u));
     asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(y));
     return (double)y;
-#else
-    return (double)(float)(1.0 / std::sqrt(std::sqrt((double)(float)u)));
-#endif
 }
 
 // The four polynomials of one interval at s, degree DEG.
 template <int DEG>
-__host__ __device__ __forceinline__ void gh_poly(const double (&t)[4][DEG + 1], double s, double (&v)[4]) {
+__device__ __forceinline__ void gh_poly(const double (&t)[4][DEG + 1], double s, double (&v)[4]) {
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) v[ch] = t[ch][DEG];
 #pragma unroll
@@ -163,7 +153,7 @@ __host__ __device__ __forceinline__ void gh_poly(const double (&t)[4][DEG + 1], 
 }
 
 // Sine and cosine on [-pi/4, pi/4] (Taylor, truncation below 7e-17), turned by n pi/2.
-__host__ __device__ __forceinline__ void gh_sincos_quadrant(double r, int n, double &sn, double &cs) {
+__device__ __forceinline__ void gh_sincos_quadrant(double r, int n, double &sn, double &cs) {
     const double z = r * r;
     double ps = -1.0 / 1307674368000.0, pc = 1.0 / 20922789888000.0;
     ps = fma(ps, z, 1.0 / 6227020800.0);
@@ -185,28 +175,6 @@ __host__ __device__ __forceinline__ void gh_sincos_quadrant(double r, int n, dou
     cs = ((n + 1) & 2) ? -b : b;
 }
 
-#ifndef __CUDA_ARCH__
-static inline long long gh_bits(double v) {
-    long long b;
-    __builtin_memcpy(&b, &v, sizeof(b));
-    return b;
-}
-#endif
-
-__host__ __device__ __forceinline__ int gh_low_word(double v) {
-#ifdef __CUDA_ARCH__
-    return __double2loint(v);
-#else
-    return (int)gh_bits(v);
-#endif
-}
-__host__ __device__ __forceinline__ int gh_high_word(double v) {
-#ifdef __CUDA_ARCH__
-    return __double2hiint(v);
-#else
-    return (int)(gh_bits(v) >> 32);
-#endif
-}
 // High words of the interval bounds (u is compared by them: no FP64 comparison per point; a
 // bound's low word is 0, so the comparisons are exact).
 #define GH_HI_MIN 0x39b00000  // 2^-100
@@ -218,7 +186,7 @@ __host__ __device__ __forceinline__ int gh_high_word(double v) {
 #define GH_HI_D 0x40220000    // 3^2
 
 // s = u^{-1/4}, inv = 1/x, x = sqrt(u).
-__host__ __device__ __forceinline__ void gh_roots(double u, double &s, double &inv, double &x) {
+__device__ __forceinline__ void gh_roots(double u, double &s, double &inv, double &x) {
     // e = 1 - u s^4 of the estimate (below 1e-6), then (1 - e)^{-1/4} to e^2
     s = gh_fourth_root_estimate(u);
     const double s2 = s * s;
@@ -230,17 +198,17 @@ __host__ __device__ __forceinline__ void gh_roots(double u, double &s, double &i
 }
 
 // Phase x - pi/4 = n pi/2 + r: n rounded by the 1.5 2^52 shift, r = x - (2n + 1) pi/4.
-__host__ __device__ __forceinline__ void gh_phase(double x, double &sn, double &cs) {
+__device__ __forceinline__ void gh_phase(double x, double &sn, double &cs) {
     const double shift = 6755399441055744.0;
     const double t = fma(x, 0.63661977236758134308, -0.5) + shift;
     const double m = fma(2.0, t - shift, 1.0);
     double r = fma(-m, 0.78539816339744830962, x);
     r = fma(-m, 3.0616169978683829431e-17, r);
-    gh_sincos_quadrant(r, gh_low_word(t), sn, cs);
+    gh_sincos_quadrant(r, __double2loint(t), sn, cs);
 }
 
 // The Hankel pair from modulus polynomials v, s = x^{-1/2}, inv = 1/x and the phase.
-__host__ __device__ __forceinline__ void gh_combine(const double (&v)[4], double s, double inv, double sn, double cs,
+__device__ __forceinline__ void gh_combine(const double (&v)[4], double s, double inv, double sn, double cs,
                                                     double2 &g, double2 &h) {
     // g = (j/4) sqrt(2/(pi x)) (cos - j sin)(P0 - j Q0); H1 carries another factor j
     const double A = 0.19947114020071633897 * s;  // sqrt(2/pi)/4
@@ -251,15 +219,15 @@ __host__ __device__ __forceinline__ void gh_combine(const double (&v)[4], double
 }
 
 // Sine and cosine of x, |x| < 2^30: x = n pi/2 + r in two parts, then the polynomials.
-__host__ __device__ __forceinline__ void gh_sincos(double x, double &sn, double &cs) {
+__device__ __forceinline__ void gh_sincos(double x, double &sn, double &cs) {
     const double shift = 6755399441055744.0;
     const double t = fma(x, 0.63661977236758134308, shift), m = t - shift;
     double r = fma(-m, 1.57079632679489661923, x);
     r = fma(-m, 6.1232339957367658862e-17, r);
-    gh_sincos_quadrant(r, gh_low_word(t), sn, cs);
+    gh_sincos_quadrant(r, __double2loint(t), sn, cs);
 }
 
-__host__ __device__ __noinline__ static void hankel_pair_library(double u, double2 &g, double2 &h) {
+__device__ __noinline__ static void hankel_pair_library(double u, double2 &g, double2 &h) {
     const double x = sqrt(u);
     g = make_double2(0.25 * y0(x), 0.25 * j0(x));
     h = make_double2(0.25 * y1(x) / x, 0.25 * j1(x) / x);
@@ -267,8 +235,8 @@ __host__ __device__ __noinline__ static void hankel_pair_library(double u, doubl
 
 // g = (j/4) H0^(2)(x), h = (j/4) H1^(2)(x) / x, x = sqrt(u).  Outside 2^-100 <= u < 2^93 (the
 // FP32 range of the root estimate, exact phase multiples) the library functions.
-__host__ __device__ __forceinline__ void hankel_pair(double u, double2 &g, double2 &h) {
-    const int hi = gh_high_word(u);
+__device__ __forceinline__ void hankel_pair(double u, double2 &g, double2 &h) {
+    const int hi = __double2hiint(u);
     if (hi < GH_HI_MIN || hi >= GH_HI_MAX) {
         hankel_pair_library(u, g, h);
         return;
@@ -279,16 +247,16 @@ __host__ __device__ __forceinline__ void hankel_pair(double u, double2 &g, doubl
         const double y = inv * inv;
         constexpr double yz = 1.0 / (GH_XZ * GH_XZ), ya = 1.0 / (GH_XA * GH_XA), yb = 1.0 / (GH_XB * GH_XB),
                          yc = 1.0 / (GH_XC * GH_XC), yd = 1.0 / (GH_XD * GH_XD);
-        if (hi >= GH_HI_Z) gh_poly<GH_DEG_Z>(GH_TAB.z, fma(y, 2.0 / yz, -1.0), v);
-        else if (hi >= GH_HI_A) gh_poly<GH_DEG_A>(GH_TAB.a, fma(y, 2.0 / (ya - yz), -(ya + yz) / (ya - yz)), v);
-        else if (hi >= GH_HI_B) gh_poly<GH_DEG_B>(GH_TAB.b, fma(y, 2.0 / (yb - ya), -(yb + ya) / (yb - ya)), v);
-        else if (hi >= GH_HI_C) gh_poly<GH_DEG_C>(GH_TAB.c, fma(y, 2.0 / (yc - yb), -(yc + yb) / (yc - yb)), v);
-        else gh_poly<GH_DEG_C>(GH_TAB.d, fma(y, 2.0 / (yd - yc), -(yd + yc) / (yd - yc)), v);
+        if (hi >= GH_HI_Z) gh_poly<GH_DEG_Z>(c_hankel.z, fma(y, 2.0 / yz, -1.0), v);
+        else if (hi >= GH_HI_A) gh_poly<GH_DEG_A>(c_hankel.a, fma(y, 2.0 / (ya - yz), -(ya + yz) / (ya - yz)), v);
+        else if (hi >= GH_HI_B) gh_poly<GH_DEG_B>(c_hankel.b, fma(y, 2.0 / (yb - ya), -(yb + ya) / (yb - ya)), v);
+        else if (hi >= GH_HI_C) gh_poly<GH_DEG_C>(c_hankel.c, fma(y, 2.0 / (yc - yb), -(yc + yb) / (yc - yb)), v);
+        else gh_poly<GH_DEG_C>(c_hankel.d, fma(y, 2.0 / (yd - yc), -(yd + yc) / (yd - yc)), v);
         double sn, cs;
         gh_phase(x, sn, cs);
         gh_combine(v, s, inv, sn, cs, g, h);
     } else {
-        gh_poly<GH_DEG_E>(GH_TAB.e, fma(u, 2.0 / (GH_XD * GH_XD), -1.0), v);
+        gh_poly<GH_DEG_E>(c_hankel.e, fma(u, 2.0 / (GH_XD * GH_XD), -1.0), v);
         const double l = 0.31830988618379067154 * log(0.25 * u);  // (2/pi) ln(x/2)
         g = make_double2(0.25 * fma(l, v[0], v[2]), 0.25 * v[0]);
         h = make_double2(0.25 * (fma(l, v[1], v[3]) - 0.63661977236758134308 * (inv * inv)), 0.25 * v[1]);
@@ -298,7 +266,7 @@ __host__ __device__ __forceinline__ void hankel_pair(double u, double2 &g, doubl
 // Two arguments at once: where both lie at x >= 25 (most points of a large body) the two
 // evaluations run interleaved and share every coefficient load; else one after the other.
 __device__ __forceinline__ void hankel_pair2(const double (&u)[2], double2 (&g)[2], double2 (&h)[2]) {
-    const int hi0 = gh_high_word(u[0]), hi1 = gh_high_word(u[1]);
+    const int hi0 = __double2hiint(u[0]), hi1 = __double2hiint(u[1]);
     const int lo = min(hi0, hi1), top = max(hi0, hi1);
     if (lo >= GH_HI_A && top < GH_HI_MAX) {
         double s[2], inv[2], x[2], v[2][4], sn[2], cs[2];
