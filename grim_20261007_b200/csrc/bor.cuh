@@ -76,7 +76,8 @@ __device__ __forceinline__ BorPt bor_point(const double *nodes, int e, double s,
     return p;
 }
 
-// Far-pair xi sample count (multiple of 32, so that sin(x) = cos(x - pi/2) is a table shift).
+// Far-pair xi sample count: a multiple of 32, of which the double fold needs four (xi = pi/2 is a
+// sample and its own partner).
 __device__ __forceinline__ int bor_nxi(double k, double rp, double rq, double r0, int mmax) {
     const double c = sqrt(rp * rq);
     const double v = 1.5 * (2.0 * k * c + mmax + 2) + 40.0 * c / fmax(r0, 1e-300) + 16.0;

@@ -849,8 +849,8 @@ __device__ __forceinline__ int gal_tile_order(int ne, int e0, int f0, const GalE
 // values d_0, d_1 is d_0 phi_a phi_0 + d_1 phi_a phi_1): six sums a point instead of eight
 // products and eight sums, and no cancellation (every weight is positive).
 // The running sums wait in shared memory, so that 128 registers hold two interleaved points
-// (each coefficient load serves both).  N = 2048, TE (8 x 8 points): 1.37 ms at 59 % of the
-// FP64 pipe, against 2.50 ms with four library Bessel calls a point.
+// (each coefficient load serves both).  N = 2048, TE: 1.25 ms at 58 % of the FP64 pipe (1.37 with 8
+// x 8 points everywhere, 2.50 with four library Bessel calls a point).
 // LANES threads share a pair, taking every LANES-th observation point each: 8 where one
 // thread per pair would leave the chip idle (N = 333: 0.10 ms, 0.80 ms with one), else 1.
 template <int POL, typename C, int LANES>

@@ -3021,7 +3021,7 @@ static int bor_moments_launch(grim_context *h, int ne, const double *nodes, cons
                                     h->stream));
     GRIM_CHECK_CUDA(cudaMemcpyAsync(p_pairs, pairs.data(), pairs.size() * sizeof(int4), cudaMemcpyHostToDevice,
                                     h->stream));
-    // eight warps, or as many as leave room for the item's moments (128 orders: six)
+    // eight warps, or as many as leave room for the item's moments (128 orders: seven)
     auto near_bytes = [&](int warps) {
         return sizeof(double2) * ((size_t)warps * bor_near_area(nm, NV, bor_near_blocks(nm, MB)) + (size_t)nm * nsl) +
                sizeof(double) * warps * nsl + sizeof(BorGauss);
@@ -3075,7 +3075,8 @@ extern "C" int grim_bor_moments(grim_handle_t h, int ne, const double *nodes, do
                                     h->stream));
     // per-launch profiling: the kernels' spans start here, not at the caller's host work
     if (h->profiling) grim_prof_mark(h, "bor_upload", 0, 0);
-    // a multiple of 32 keeps the shared-memory sections after the sample table 16-byte aligned
+    // the far rule folds its samples at xi = pi/2: every count, the cap too, is a multiple of four
+    // (bor_nxi rounds to 32)
     const int cap = std::min(BOR_MAX_NXI, (std::max(32, nxi_max) + 31) / 32 * 32);
     const bool three = bor_mb(mmax + 2) == 3;
     auto launch = mom_k ? (three ? bor_moments_launch<true, 3> : bor_moments_launch<true, 4>)

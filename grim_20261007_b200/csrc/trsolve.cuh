@@ -10,12 +10,14 @@
 //      rows by every other group of four k-steps (eight warps left half the tensor pipe idle:
 //      two a scheduler do not cover the instructions between the MMAs).  Fragments come
 //      straight from L2 -- eight consecutive rows of a column are one 128-byte line, read once
-//      per strip -- two groups ahead; the solved rows, read by eight warps, from L1;
-//      meanwhile the diagonal block arrives in shared memory with cp.async;
+//      per strip by one warp -- two groups ahead; the solved rows, each read by the eight warps
+//      of its half of the groups, from L1; meanwhile the diagonal block arrives in shared memory
+//      with cp.async;
 //   2. the 64-row substitution, one warp per column, two rows per lane;
 //   3. X_i to global memory, where step 1 of the next block reads it.
 // Bound by the FP64 tensor pipe of the SMs that have a strip (8 n^2 x 8 / 2 flops a strip and
-// triangle) and the substitution chain (about 4 us a block).  getrs, both triangles with the
+// triangle; 51 % of it over the whole chip at 90 strips) and the substitution chain (about 4 us a
+// block).  getrs, both triangles with the
 // interchanges, blocked launches before -> strips: N = 400, 722 columns 0.53 -> 0.18 ms;
 // N = 1024, 361 1.30 -> 0.61 ms; N = 2048, 720 3.40 -> 1.99 ms; N = 4096, 720 9.5 -> 7.2 ms.
 #pragma once
@@ -30,8 +32,7 @@
 #define TRS_LDT (NB + 1)
 #define TRS_SMEM ((size_t)(NB * TRS_LDT + 2 * TRS_COLS * TRS_LDT + NB) * sizeof(double2))
 
-// A read-once element of the factor: not kept in L1 (the solved rows, read by all eight warps,
-// are).
+// A read-once element of the factor: not kept in L1 (the solved rows, read by eight warps, are).
 __device__ __forceinline__ double2 trs_stream(const double2 *p) {
     double2 v;
     asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));

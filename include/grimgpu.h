@@ -86,8 +86,10 @@ typedef struct grim_solve_info {
     int pivoted_panels;          /* panels that needed row interchanges (0 = diagonal pivots certified) */
     int precision_mode;
     int info;                    /* LAPACK-style: >0 = U(info,info) exactly zero      */
-    double ms_factor;            /* device time of the factorization                 */
-    double ms_solve;             /* device time of the triangular solves + refinement */
+    double ms_factor;            /* device time of the factorization, with the forward
+                                    elimination where that runs beside it             */
+    double ms_solve;             /* device time of the remaining triangular solves and
+                                    the refinement                                    */
 } grim_solve_info;
 
 /* ---- context ------------------------------------------------------------------ */
