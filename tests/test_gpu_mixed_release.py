@@ -47,7 +47,7 @@ def test_iterates_in_the_last_decade_are_corrected_once_more(n, nrhs):
                                             (2.4875701825175005, 0.7986149919634109, 0.3880252084505901, 0.6811946510427173)])
 def test_large_mixed_amplitudes_are_those_of_the_fp64_solve(p, a, b, phase):
     """An accepted backward error of at most 1e-11, or 1e-10 and another correction, leaves at
-    most 34 times 1e-11 in the amplitudes, the slices of the residual 5e-10."""
+    most 34 times 1e-11 in the amplitudes, the slices of the residual the rest."""
     from grim_20261007_b200.twod import operators as ops
     from grim_20261007_b200.twod.galerkin import GalerkinBody
     n = 4099
