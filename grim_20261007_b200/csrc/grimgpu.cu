@@ -2780,11 +2780,17 @@ static int far_block_host(bool fresh, int64_t mb, int64_t nb, int q, int width, 
                                double *acc_kt) {
     if (!far_args_ok(mb, nb, q, width, want_s, want_k, mirrored, intervals, degree, acc_s, acc_k, acc_kt)) return 3;
     if (mb == 0 || nb == 0) return 0;
-    static thread_local grim_context *h = nullptr;
+    // the thread's handle, given back (streams, device workspace, pinned slots) when it ends
+    struct ThreadHandle {
+        grim_context *h = nullptr;
+        ~ThreadHandle() { grim_destroy(h); }
+    };
+    static thread_local ThreadHandle own;
+    grim_context *&h = own.h;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return GRIM_ERR_CUDA;
     if (!h || h->device != dev) {
-        if (h) grim_destroy(h);
+        grim_destroy(h);
         h = nullptr;
         GRIM_TRY(grim_create(dev, &h));
     }
