@@ -58,12 +58,13 @@ static bool stage_ready(grim_context *h) {
 }
 
 // The copies of `list`, in stream order on the handle's stream, up (host to device; returns when
-// the host buffers have been read) or down (returns when they have been written).
+// the host buffers have been read) or down (returns when they have been written).  On
+// cudaStreamPerThread, which names another stream on every thread, the plain copies.
 static int stage_copy(grim_context *h, const std::vector<HostCopy> &list, bool up) {
     size_t total = 0;
     for (const HostCopy &c : list) total += c.bytes;
     const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-    if (total < STAGE_MIN || !stage_ready(h)) {
+    if (total < STAGE_MIN || h->stream == cudaStreamPerThread || !stage_ready(h)) {
         for (const HostCopy &c : list)
             GRIM_CHECK_CUDA(cudaMemcpyAsync(up ? c.device : c.host, up ? c.host : c.device, c.bytes, kind, h->stream));
         GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));

@@ -95,6 +95,34 @@ def test_row_major_systems_take_millions_of_columns():
     assert np.max(np.abs(a @ x - b)) <= 1e-14 * np.max(np.abs(b))
 
 
+@pytest.mark.parametrize('rows', [False, True])
+def test_dense_systems_on_the_per_thread_stream(rows):
+    """cudaStreamPerThread (handle value 2) is another stream on every thread: copies from a team of
+    threads would not be ordered with the solve."""
+    import ctypes
+    from grim_20261007_b200 import _lib
+    lib = _lib.load()
+    n, nrhs = 700, 90
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * n ** 0.5 * np.eye(n)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    h, info = ctypes.c_void_p(), ctypes.c_int(-1)
+    _lib.check(lib.grim_create(0, ctypes.byref(h)))
+    try:
+        _lib.check(lib.grim_set_stream(h, ctypes.c_void_p(2)))
+        if rows:
+            x = np.empty_like(b)
+            _lib.check(lib.grim_zgesv_rowmajor(h, n, nrhs, a.ctypes.data, b.ctypes.data, x.ctypes.data, _lib.PREC_FP64,
+                                               ctypes.byref(info)))
+        else:
+            af, x = np.asfortranarray(a), np.asfortranarray(b)
+            _lib.check(lib.grim_zgesv_batched(h, n, nrhs, af.ctypes.data, n, x.ctypes.data, n, _lib.PREC_FP64,
+                                              ctypes.byref(info)))
+    finally:
+        lib.grim_destroy(h)
+    assert np.max(np.abs(a @ x - b)) < 1e-14 * (np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x)))
+
+
 @pytest.mark.parametrize('rows, cols', [(3, 2), (130, 131), (181, 182), (300, 257)])
 def test_far_block_from_zero_equals_accumulating(rows, cols):
     """Fresh accumulators equal sums into zeros; sums into other values keep them."""
