@@ -2827,8 +2827,8 @@ static int far_block_host(bool fresh, int64_t mb, int64_t nb, int q, int width, 
     if (with_kt) acc.push_back({d_akt, acc_kt, acc_bytes});
     if (!fresh) in.insert(in.end(), acc.begin(), acc.end());
     GRIM_TRY(stage_copy(h, in, true));
-    if (fresh)
-        for (const HostCopy &c : acc) GRIM_CHECK_CUDA(cudaMemsetAsync(c.device, 0, c.bytes, h->stream));
+    if (fresh)  // the accumulators lie one after the other
+        GRIM_CHECK_CUDA(cudaMemsetAsync(acc[0].device, 0, acc.size() * acc_bytes, h->stream));
     const int s = grim_far_block(h, mb, nb, q, width, d_op, d_sp, d_qw, d_phi, d_on, d_sn, d_far, obs_normal_deriv,
                                  want_s, want_k, mirrored, k_re, k_im, intervals, d_b, degree, d_c,
                                  want_s ? d_as : nullptr, want_k ? d_ak : nullptr, with_kt ? d_akt : nullptr);

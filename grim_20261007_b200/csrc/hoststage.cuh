@@ -19,7 +19,12 @@
 #define STAGE_CHUNK ((size_t)1 << 20)
 #define STAGE_THREADS 8
 #define STAGE_SLOTS (2 * STAGE_THREADS)
-#define STAGE_MIN ((size_t)2 << 20)  // below it the plain copy (0.2 ms) costs less than the threads
+// From these totals on the threads cost less than the plain copy: up, from buffers that are in
+// place (64 x 2000, 2.1 MB 0.89 ms plain, 0.95 staged; 300 x 300, 2.9 MB 1.50, 1.54; 450 x 181, 4.5
+// MB 1.96, 1.83; 900 x 1, 13 MB 3.56, 3.02), and down, into fresh pages (far blocks of 1.9 MB 0.52,
+// 0.48; 3.1 MB 0.73, 0.56; 12.6 MB 2.07, 1.02).
+#define STAGE_MIN_UP ((size_t)4 << 20)
+#define STAGE_MIN_DOWN ((size_t)2 << 20)
 
 struct HostCopy {
     void *device, *host;
@@ -57,17 +62,17 @@ static bool stage_ready(grim_context *h) {
     return true;
 }
 
-// The copies of `list`, in stream order on the handle's stream, up (host to device; returns when
-// the host buffers have been read) or down (returns when they have been written).  On
+// The copies of `list`, in stream order on the handle's stream, up (host to device; the host
+// buffers are read in stream order at the latest) or down (returns when they have been written).  On
 // cudaStreamPerThread, which names another stream on every thread, the plain copies.
 static int stage_copy(grim_context *h, const std::vector<HostCopy> &list, bool up) {
     size_t total = 0;
     for (const HostCopy &c : list) total += c.bytes;
     const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-    if (total < STAGE_MIN || h->stream == cudaStreamPerThread || !stage_ready(h)) {
+    if (total < (up ? STAGE_MIN_UP : STAGE_MIN_DOWN) || h->stream == cudaStreamPerThread || !stage_ready(h)) {
         for (const HostCopy &c : list)
             GRIM_CHECK_CUDA(cudaMemcpyAsync(up ? c.device : c.host, up ? c.host : c.device, c.bytes, kind, h->stream));
-        GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));
+        if (!up) GRIM_CHECK_CUDA(cudaStreamSynchronize(h->stream));
         return GRIM_OK;
     }
     std::vector<HostCopy> chunks;

@@ -1,5 +1,5 @@
-"""Host-buffer entry points around the sizes where their copies change: below 2 MiB one plain
-copy, above it 1 MiB chunks through the handle's pinned slots on several threads; row-major
+"""Host-buffer entry points around the sizes where their copies change: below 4 MiB up and 2 MiB
+down one plain copy, above it 1 MiB chunks through the handle's pinned slots on several threads; row-major
 systems are transposed on the device."""
 import numpy as np
 import pytest
@@ -31,6 +31,18 @@ def test_dense_hook_takes_every_layout(n, nrhs, layout):
     assert x.flags.c_contiguous if bl.flags.c_contiguous else x.flags.f_contiguous
     v, _name = _solve_dense_gpu(al, np.ascontiguousarray(b[:, 0]))
     assert v.shape == (n,) and np.max(np.abs(v - x[:, 0])) <= 1e-13 * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize('n, nrhs', [(511, 1), (512, 1), (500, 262), (500, 263)])
+@pytest.mark.parametrize('order', ['C', 'F'])
+def test_dense_hook_on_both_sides_of_the_staged_copies(n, nrhs, order):
+    """4 MiB of matrix and right-hand sides up, 2 MiB of solution down."""
+    from grim_20261007_b200.twod.solver import _solve_dense_gpu
+    rng = np.random.default_rng(n + nrhs)
+    a = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 3.0 * n ** 0.5 * np.eye(n)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    x, _name = _solve_dense_gpu(np.array(a, order=order), np.array(b, order=order))
+    assert np.max(np.abs(a @ x - b)) < 1e-14 * (np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x)))
 
 
 @pytest.mark.parametrize('n, nrhs', [(2, 2600), (16, 300), (16, 310), (60, 70), (60, 2500), (121, 1), (122, 1)])
