@@ -1918,8 +1918,9 @@ static int mixed_refine(grim_context *h, int n, int nrhs, const TA *Ares, int64_
             // amplitudes, 34 times the backward error, and two builds that differ by rounding
             // 3e-9 apart.  In the target's last decade the correction of the residual in hand
             // goes in too (each takes off a factor of 20 or more there): 1.5e-10 in the median of 120
-            // such bodies, 9e-10 at most, where the residual's six slices end.
-            if (berr_test && measure > 0.1 * tol && steps < max_iter) {
+            // such bodies, 9e-10 at most, where the residual's six slices end.  A matrix that is itself
+            // complex64 (6e-8 an entry) stands for no solution that closely: its iterates stay.
+            if (sizeof(TA) == sizeof(double2) && berr_test && measure > 0.1 * tol && steps < max_iter) {
                 GRIM_TRY(correct());
                 GRIM_TRY(tc_err_check(h, "mixed-precision solve"));
             }

@@ -240,9 +240,10 @@ int grim_backward_error_noalloc(grim_handle_t h, int n, int nrhs, const void *A,
  * reference linalg/refined_lu.py:25-61.  GRIM_PREC_MIXED_BERR: the same refinement
  * stopping when the normwise backward error |r| / (|A| |x| + |b|) of every column is
  * <= tol (the form of test LAPACK's zcgesv uses), for callers whose accuracy target
- * is a backward error (the RCS solves); an iterate above a tenth of tol takes the
- * correction of its residual as well before it is returned (at most max_iter corrections in
- * all; the statistics then give the backward error before that one).  A is preserved.
+ * is a backward error (the RCS solves); with a complex128 A an iterate above a tenth of
+ * tol takes the correction of its residual as well before it is returned (at most max_iter
+ * corrections in all; the statistics then give the backward error before that one).  A is
+ * preserved.
  * info: LAPACK-style.  stats may be NULL.  GRIM_PREC_STATIC_PIVOT or GRIM_PREC_PARTIAL_PIVOT
  * or-ed into the mode picks the factorization's pivot mode (GRIM_PIVOT_STATIC /
  * GRIM_PIVOT_PARTIAL; the default is CERTIFIED); with static pivots the refinement guards the

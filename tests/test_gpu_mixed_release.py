@@ -8,15 +8,16 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip('torch')
 
 
-def _solve(a, b, tol, max_iter):
+def _solve(a, b, tol, max_iter, complex64=False):
     from grim_20261007_b200 import _lib
     from grim_20261007_b200.device import context, ptr, to_device_colmajor, to_host_matrix
     ctx = context()
     n, nrhs = b.shape
-    at, bt = (to_device_colmajor(v, torch.complex128) for v in (a, b))
+    at, bt = to_device_colmajor(a, torch.complex64 if complex64 else torch.complex128), to_device_colmajor(b, torch.complex128)
+    args = (None, n, ptr(at), n) if complex64 else (ptr(at), n, None, 0)
     info, st = ctypes.c_int(-1), _lib.GrimSolveInfo()
-    _lib.check(ctx.lib.grim_zgesv_mixed(ctx.h, n, nrhs, ptr(at), n, None, 0, ptr(bt), n, _lib.PREC_MIXED_BERR, tol,
-                                        max_iter, ctypes.byref(info), ctypes.byref(st)))
+    _lib.check(ctx.lib.grim_zgesv_mixed(ctx.h, n, nrhs, *args, ptr(bt), n, _lib.PREC_MIXED_BERR, tol, max_iter,
+                                        ctypes.byref(info), ctypes.byref(st)))
     x = to_host_matrix(bt)
     r = np.max(np.abs(a @ x - b), axis=0)
     den = np.max(np.sum(np.abs(a), axis=1)) * np.max(np.abs(x), axis=0) + np.max(np.abs(b), axis=0)
@@ -37,6 +38,18 @@ def test_iterates_in_the_last_decade_are_corrected_once_more(n, nrhs):
     # a target well above it, or no correction left: as it stands
     for tol, most in ((20.0 * first, 4), (2.0 * first, 0)):
         got, st = _solve(a, b, tol, most)
+        assert st.refinement_steps == 0 and 0.5 * first <= got <= 2.0 * first
+
+
+@pytest.mark.parametrize('n, nrhs', [(96, 3), (300, 40)])
+def test_iterates_of_a_complex64_matrix_stay_as_they_are(n, nrhs):
+    rng = np.random.default_rng(n)
+    a = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)) + 4.0 * n ** 0.5 * np.eye(n)).astype(np.complex64)
+    b = rng.standard_normal((n, nrhs)) + 1j * rng.standard_normal((n, nrhs))
+    first, st = _solve(a.astype(complex), b, 1.0, 4)
+    assert st.refinement_steps == 0 and 1e-9 < first < 1e-5
+    for tol in (2.0 * first, 20.0 * first):
+        got, st = _solve(a, b, tol, 4, complex64=True)
         assert st.refinement_steps == 0 and 0.5 * first <= got <= 2.0 * first
 
 
